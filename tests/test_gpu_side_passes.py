@@ -1,0 +1,52 @@
+"""The passes beside the gas step at the sizes where their work splits can go wrong: radiation over ray and
+piece counts (ray tiles of 64, lanes sharing the pieces), geometry with many pieces (per-tile piece lists),
+the renderer's persistent tiles, and the FP64 sums over one to many CTAs."""
+import numpy as np
+import pytest
+
+import campfire_b200 as cb
+from campfire_b200.fluid import load_scene
+from campfire_b200.render import Renderer, render_device
+
+pytestmark = pytest.mark.gpu
+
+
+def _scene(nx, ny, npieces, seed):
+    """A generated scene's gas with `npieces` rotated squares of its own, some touching or beyond the domain."""
+    sc = cb.generate_scene(0, nx, ny, 0.8, seed)
+    rng = np.random.default_rng(seed)
+    a = np.zeros((64, 20), np.float32)
+    H = 0.8 / nx * ny
+    for n in range(npieces):
+        a[n] = [rng.uniform(-0.05, 0.85), rng.uniform(0.0, H), rng.uniform(-3, 3), rng.uniform(0.005, 0.03), 0, 0, 0,
+                0.0 if n % 7 == 5 else 1.0, *rng.uniform(400, 1000, 4), *([0.0] * 8)]
+    sc.update(pieces=a.ravel(), npieces=npieces)
+    return sc
+
+
+def _image(sim, W, H, view):
+    import torch
+    ren = Renderer(sim)
+    rng = np.random.default_rng(3)
+    w = rng.uniform(0.001, 1.0, (64, 12)).astype(np.float32)
+    w[:, 0:4] *= 800
+    ren.writeWood(w)
+    ren.writeParams({"view": view, "exposure": 1.0, "time": 0.0})
+    img = torch.empty(H, W, 4, device="cuda")
+    render_device(sim, ren.rp, W, H, img.data_ptr(), ren.wood)
+    sim.synchronize()
+    return img.cpu().numpy()
+
+
+@pytest.mark.parametrize("view", ["photo", "temperature"])
+@pytest.mark.parametrize("W,H,npieces", [(1, 1, 1), (16, 33, 0), (47, 50, 40), (480, 497, 64)])
+def test_a_pixel_does_not_depend_on_its_image(view, W, H, npieces):
+    # the centre of pixel (x, y) is the centre of pixel (3x+1, 3y+1) of an image three times as large, to the bit
+    # (both are one correctly rounded quotient of the same number); 1440x1491 is several rounds of the CTAs
+    sc = _scene(64, 96, npieces, 11)
+    g = cb.FluidSim(0, {"nx": 64, "ny": 96, "dt": sc["dt"]}, width=0.8).init()
+    load_scene(g, sc)
+    g.step(2)
+    small, big = _image(g, W, H, view), _image(g, 3 * W, 3 * H, view)
+    g.close()
+    assert np.array_equal(small.view(np.uint32), big[1::3, 1::3].copy().view(np.uint32))
