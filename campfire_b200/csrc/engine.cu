@@ -168,6 +168,7 @@ int Engine::init(int device, int n, const int* nx, const int* ny, const double* 
   CFG_CUDA(prepare_mg_coarse(coarse_smem_));
   CFG_CUDA(prepare_coarse_factor(cf_smem_));
   CFG_CUDA(prepare_diffuse_sources());
+  CFG_CUDA(prepare_radiation());
   CFG_CUDA(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
   CFG_CUDA(cudaStreamCreateWithFlags(&body_stream_, cudaStreamNonBlocking));
   CFG_CUDA(cudaStreamCreateWithFlags(&side_stream_, cudaStreamNonBlocking));
@@ -852,7 +853,7 @@ int Engine::radiation(int s) {
   CFG_TRY(activate());
   const Scene& sc = scenes_[s];
   const int np = std::min(std::max(sc.desc.P.nPieces, 0), MAX_PIECES);
-  launch_radiation(d_scenes_, s, np * 4 + N_FLOOR, sc.nray, st());
+  launch_radiation(d_scenes_, s, sc.nx, sc.ny, np * 4 + N_FLOOR, sc.nray, st());
   CFG_CUDA(cudaGetLastError());
   return CFG_OK;
 }
