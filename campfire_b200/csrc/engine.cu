@@ -1113,7 +1113,7 @@ int Engine::info(int s, cfg_info* o) {
 int Engine::pressure_residual(int s, double* rel) {
   if (!rel) return fail(CFG_ERR_INVAL, "null output");
   CFG_TRY(activate());
-  launch_residual_norms(d_scenes_, s, d_scratch_, st());
+  launch_residual_norms(d_scenes_, s, scenes_[s].nx * scenes_[s].ny, d_scratch_, st());
   double o[2];
   CFG_CUDA(cudaMemcpyAsync(o, d_scratch_, 16, cudaMemcpyDeviceToHost, st()));
   CFG_CUDA(cudaStreamSynchronize(st()));
@@ -1123,7 +1123,7 @@ int Engine::pressure_residual(int s, double* rel) {
 int Engine::budgets(int s, double* out) {
   if (!out) return fail(CFG_ERR_INVAL, "null output");
   CFG_TRY(activate());
-  launch_budgets(d_scenes_, s, d_scratch_, st());
+  launch_budgets(d_scenes_, s, scenes_[s].nx * scenes_[s].ny, d_scratch_, st());
   CFG_CUDA(cudaMemcpyAsync(out, d_scratch_, 64, cudaMemcpyDeviceToHost, st()));
   CFG_CUDA(cudaStreamSynchronize(st()));
   return CFG_OK;

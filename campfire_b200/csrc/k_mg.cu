@@ -311,21 +311,24 @@ __global__ void __launch_bounds__(256) k_accum64(const SceneDesc* __restrict__ s
   S.p64[j * L.nx + i] += (double)L.p[j * L.pc + i];
 }
 
-// ||r||2 and ||rhs||2 of level 0 for one scene (diagnostic, one CTA)
-__global__ void __launch_bounds__(1024) k_residual_norms(const SceneDesc* __restrict__ scenes, int scene, double* out) {
-  __shared__ double red[32];
+// ||r||2 and ||rhs||2 of level 0 for one scene: each CTA leaves its two sums as partials (the
+// scene's scratch of the step's reductions, free between steps), the last one to arrive adds them in
+// order. One cell per thread and round, enough CTAs to fill the GPU: one CTA alone walked 384
+// cells per thread, one L2 round trip after another. The call at 512x768,
+// result on the host: 335 -> 31 us.
+__global__ void __launch_bounds__(256) k_residual_norms(const SceneDesc* __restrict__ scenes, int scene, double* out) {
+  __shared__ double sh[2 * 257];
   const SceneDesc& S = scenes[scene];
   const LevelDesc L = S.lev[0];
-  double vr = 0.0, vb = 0.0;
-  for (int e = threadIdx.x; e < L.nx * L.ny; e += blockDim.x) {
+  double v[2] = {0.0, 0.0};
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < L.nx * L.ny; e += gridDim.x * blockDim.x) {
     const int i = e % L.nx, j = e / L.nx;
     const double r = (double)residual(L, i, j);
     const double b = (double)L.rhs[j * L.pc + i];
-    vr += r * r; vb += b * b;
+    v[0] += r * r; v[1] += b * b;
   }
-  const double tr = block_sum(vr, red);
-  const double tb = block_sum(vb, red);
-  if (threadIdx.x == 0) { out[0] = tr; out[1] = tb; }
+  block_sum_t<2>(v, sh);
+  if (scene_reduce_n<2>(S, blockIdx.x, gridDim.x, v, sh) && threadIdx.x == 0) { out[0] = v[0]; out[1] = v[1]; }
 }
 
 // ||rhs||^2 of level 0 (FP64 mode: of rhs64); arms the pressure loop of every scene
@@ -401,8 +404,8 @@ bool pdl_enabled() { return g_pdl.load(); }
 void launch_accum64(const SceneDesc* scenes, const Work* work, int ntiles, cudaStream_t st) {
   if (ntiles > 0) k_accum64<<<ntiles, MG_TX * MG_TY, 0, st>>>(scenes, work);
 }
-void launch_residual_norms(const SceneDesc* scenes, int scene, double* out, cudaStream_t st) {
-  k_residual_norms<<<1, 1024, 0, st>>>(scenes, scene, out);
+void launch_residual_norms(const SceneDesc* scenes, int scene, int cells, double* out, cudaStream_t st) {
+  k_residual_norms<<<monitor_ctas(cells), 256, 0, st>>>(scenes, scene, out);
 }
 
 }  // namespace cfg

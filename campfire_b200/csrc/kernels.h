@@ -159,9 +159,13 @@ void launch_geometry(const SceneDesc* scenes, const Work* work, int ntiles, cuda
 void launch_radiation(const SceneDesc* scenes, int scene, int nx, int ny, int ntargets, int nray, cudaStream_t st);
 cudaError_t prepare_radiation();   // its dynamic shared memory, once per device before the first launch
 // FP64 budgets of one scene into out[8] (device)
-void launch_budgets(const SceneDesc* scenes, int scene, double* out, cudaStream_t st);
+void launch_budgets(const SceneDesc* scenes, int scene, int cells, double* out, cudaStream_t st);
 // ||r||2 and ||rhs||2 of level 0 of one scene into out[2] (device, FP64)
-void launch_residual_norms(const SceneDesc* scenes, int scene, double* out, cudaStream_t st);
+// CTAs of the one-scene FP64 sums (256 threads, a cell per thread and round): at most one per 256
+// cells, so that their partials (up to nine per CTA) fit the scene's per-tile scratch, and at
+// most four per SM, beyond which the last CTA's walk over the partials grows
+inline int monitor_ctas(int cells) { return cells < 256 * 592 ? (cells + 255) / 256 : 592; }
+void launch_residual_norms(const SceneDesc* scenes, int scene, int cells, double* out, cudaStream_t st);
 // render.wgsl's fragment stage of one scene: W x H float4 pixels, row 0 at the top
 void launch_render(const SceneDesc* scenes, int scene, const cfg_render_params& rp, const float* wood, int width,
                    int height, float* out, cudaStream_t st);

@@ -1,6 +1,8 @@
 """The passes beside the gas step at the sizes where their work splits can go wrong: radiation over ray and
 piece counts (ray tiles of 64, lanes sharing the pieces), geometry with many pieces (per-tile piece lists),
 the renderer's persistent tiles, and the FP64 sums over one to many CTAs."""
+import math
+
 import numpy as np
 import pytest
 
@@ -94,3 +96,25 @@ def test_a_pixel_does_not_depend_on_its_image(view, W, H, npieces):
     small, big = _image(g, W, H, view), _image(g, 3 * W, 3 * H, view)
     g.close()
     assert np.array_equal(small.view(np.uint32), big[1::3, 1::3].copy().view(np.uint32))
+
+
+@pytest.mark.parametrize("nx,ny", [(2, 2), (15, 17), (16, 32), (224, 320), (512, 768)])
+def test_monitor_sums(oracle_mod, nx, ny):
+    g, o = _pair(oracle_mod, nx, ny, 3, 5)
+    g.step(1)
+    T, Y = g.readBuffer("T").astype(np.float64), g.readBuffer("Y").astype(np.float64).reshape(-1, 4)
+    G, SQ = g.readBuffer("cellG").reshape(-1, 2), g.readBuffer("SQ").astype(np.float64).reshape(-1, 2)
+    gas = ~((G[:, 0] < 0) & (G[:, 1].view(np.uint32) != 0xffffffff))
+    p = g.params
+    dx2 = float(np.float32(p["dx"])) ** 2
+    m = p["rhoAmb"] * p["Tamb"] / T[gas] * dx2
+    total = lambda v: math.fsum(v.tolist())   # noqa: E731  (correctly rounded)
+    want = [total(m), total(m * p["cp"] * T[gas]), *(total(m * Y[gas, k]) for k in range(4)),
+            total(SQ[gas, 1]) * dx2, T[gas].max()]
+    # the same terms added in another order, in FP64: partial sums of at most ~1e3 terms of one sign
+    assert np.allclose(g.budgets(), want, rtol=1e-12, atol=1e-300)
+    assert np.array_equal(g.budgets(), g.budgets())
+    o.copy_state_from(g)
+    a, b = g.pressure_residual(), o.pressure_residual()
+    assert abs(a - b) <= 1e-9 * max(abs(b), 1e-12)
+    g.close()
