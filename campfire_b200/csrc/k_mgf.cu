@@ -660,6 +660,7 @@ namespace {
 constexpr int CB_THREADS = 512;
 constexpr int kStagedInverseMax = 128;   // coarsest unknowns whose inverse (<= 64 KB) is staged in shared memory
 constexpr int CB_WARPS = CB_THREADS / 32;
+constexpr int SWEEP_M = 6;              // largest coarsest level of the one-warp sweeps: 12 rows per lane
 constexpr int COARSEST_SCRATCH = 0;     // the coarsest keeps its stencils in registers
 using namespace mgc;
 
@@ -840,7 +841,69 @@ __device__ __forceinline__ void cb_down(const CbCtx c, int l) {
     }
   __syncthreads();
 }
+// The 120 red-black sweeps (pressure.wgsl:132-156) in the registers of one warp, for levels up to
+// 32 cells wide: lane (g, i) owns column i of the 2 M rows from 2 M g on, as M pairs of rows with
+// one cell of each colour. A colour pass reads the other colour only: the west and east
+// neighbours by shuffles from the lanes beside (the same pair of rows), the south and north ones
+// from the lane's own registers, at the ends of its rows from the lanes below and above. Bound
+// by the latency of the 240 dependent passes: one shuffle and one cell's arithmetic each, where
+// the block's pass (coarsest_update, kept for wider levels) adds a store to shared memory, a
+// barrier and loads. A missing neighbour's coefficient is zero and a cell without open faces has
+// zeros throughout, which leaves the sums' bits as they are.
+// Not inlined: its registers are its own, one call per coarsest solve.
+// The block of a 32x48 scene (8x12 coarsest): 31.3 -> 22.9 us, i.e. ~93 -> 58 ns per pass.
+template <int M>
+__device__ __noinline__ void sweeps_warp(float* smem, const LvO& o) {
+  const LvS L = lvs_at(smem, o);
+  const int lane = threadIdx.x & 31, ng = fdiv(32, L.mnx), g = fdiv(lane, L.mnx), i = lane - g * L.nx;
+  float w[2][M], e[2][M], so[2][M], no[2][M], rh[2][M], di[2][M], rc[2][M], p[2][M];
+  #pragma unroll
+  for (int c = 0; c < 2; c++)
+    #pragma unroll
+    for (int m = 0; m < M; m++) {
+      const int j = 2 * (g * M + m) + ((i + c) & 1);
+      w[c][m] = e[c][m] = so[c][m] = no[c][m] = rh[c][m] = di[c][m] = rc[c][m] = p[c][m] = 0.f;
+      if (g >= ng || j >= L.ny) continue;
+      const CCell q = coarsest_cell(L, j * L.nx + i);
+      if (!(q.diag > 0.f)) continue;
+      if (q.hw) w[c][m] = q.w;
+      if (q.he) e[c][m] = q.e;
+      if (q.hs) so[c][m] = q.s;
+      if (q.hn) no[c][m] = q.n;
+      rh[c][m] = q.rh; di[c][m] = q.diag; rc[c][m] = q.rcp;
+    }
+  const bool odd[2] = {(i & 1) != 0, (i & 1) == 0};   // colour c's cell is the upper row of its pair
+  #pragma unroll 1
+  for (int it = 0; it < 120; it++)
+    #pragma unroll
+    for (int c = 0; c < 2; c++) {
+      float (&q)[M] = p[1 - c];
+      const float below = __shfl_sync(0xffffffffu, q[M - 1], lane - L.nx), above = __shfl_sync(0xffffffffu, q[0], lane + L.nx);
+      #pragma unroll
+      for (int m = 0; m < M; m++) {
+        const float pw = __shfl_up_sync(0xffffffffu, q[m], 1), pe = __shfl_down_sync(0xffffffffu, q[m], 1);
+        const float ps = odd[c] ? q[m] : (m > 0 ? q[m > 0 ? m - 1 : 0] : below);
+        const float pn = odd[c] ? (m < M - 1 ? q[m < M - 1 ? m + 1 : m] : above) : q[m];
+        float off = 0.f;
+        off += w[c][m] * pw;
+        off += e[c][m] * pe;
+        off += so[c][m] * ps;
+        off += no[c][m] * pn;
+        p[c][m] = div_by_rcp(off - rh[c][m], di[c][m], rc[c][m]);
+      }
+    }
+  #pragma unroll
+  for (int c = 0; c < 2; c++)
+    #pragma unroll
+    for (int m = 0; m < M; m++) {
+      const int j = 2 * (g * M + m) + ((i + c) & 1);
+      if (g < ng && j < L.ny) L.p[j * L.pc + i] = p[c][m];
+    }
+}
 // the coarsest level's solve (its p overwritten: the inverse's product, or sweeps from zero)
+// WARP: with the one-warp sweeps (the call costs the W tail's instance, whose coarsest solve appears
+// twice, 560 bytes of spill: it keeps the block's passes)
+template <bool WARP>
 __device__ __forceinline__ void cb_coarsest(const CbCtx c) {
   float* const smem = c.smem;
   const LvO* const lvo = c.lvo;
@@ -891,7 +954,16 @@ __device__ __forceinline__ void cb_coarsest(const CbCtx c) {
       const LvS L = lvs_at(smem, lvo[nl - 1]);
       const int npair = (L.nx * L.ny + 1) >> 1;
       const int nthr = (npair + 31) & ~31;
-      if ((int)threadIdx.x < nthr) {
+      // pairs of rows a lane of the one-warp form owns
+      const int rows = L.nx <= 32 ? fdiv(32, L.mnx) * 2 : 0;
+      const int M = rows > 0 ? (L.ny + rows - 1) / rows : SWEEP_M + 1;
+      if (WARP && M <= SWEEP_M) {
+        if (warp == 0) {
+          if (M <= 2) sweeps_warp<2>(smem, lvo[nl - 1]);
+          else if (M <= 4) sweeps_warp<4>(smem, lvo[nl - 1]);
+          else sweeps_warp<SWEEP_M>(smem, lvo[nl - 1]);
+        }
+      } else if ((int)threadIdx.x < nthr) {
         const CCell a = coarsest_cell(L, 2 * threadIdx.x), b = coarsest_cell(L, 2 * threadIdx.x + 1);
         if (a.act) L.p[a.kp] = 0.f;
         if (b.act) L.p[b.kp] = 0.f;
@@ -1052,11 +1124,11 @@ __global__ void __launch_bounds__(CB_THREADS) k_mg_coarse(const SceneDesc* __res
   // from its p and restricted again (its rhs stays) and the coarsest solved again. Straight-line
   // code: the visits keep their registers to themselves.
   for (int l = lc; l < nl - 1; l++) cb_down(cbx, l);
-  cb_coarsest(cbx);
+  cb_coarsest<!WT>(cbx);
   if (WT && S.lw == nl - 3 && nl - 3 >= lc) {
     cb_up(cbx, nl - 2);
     cb_down(cbx, nl - 2);
-    cb_coarsest(cbx);
+    cb_coarsest<!WT>(cbx);
   }
   for (int l = nl - 2; l >= lc; l--) cb_up(cbx, l);
   // ---- write level lc back; when the block covers level 0, finish the cycle here
