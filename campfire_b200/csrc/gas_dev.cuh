@@ -238,6 +238,16 @@ struct VField {
   }
 };
 
+// floor(x) as an integer and the fraction x - floor(x): x + 1.5 2^23 rounded down has an ulp of 1 for
+// |x| < 2^22, so its low bits hold the floor and subtracting the constant again gives it as a
+// float, exactly; three full-rate operations where floorf and the conversion take two of a
+// sixteenth. Beyond that range (or for a NaN) the integer lies outside every grid, where the
+// samplers read the boundary values.
+__device__ __forceinline__ int floor_frac(float x, float& frac) {
+  const float y = __fadd_rd(x, 12582912.f);
+  frac = x - (y - 12582912.f);
+  return __float_as_int(y) - 0x4b400000;
+}
 // s_<name>: bilinear at g - off (cell units); off = (0.5,0.5) C, (0,0.5) U, (0.5,0) V
 // the four corners of the 2x2 block at (i, j), directly when the field allows it
 template <class F, class T>
@@ -247,38 +257,20 @@ __device__ __forceinline__ void corners(const F& f, int i, int j, T& A, T& C, T&
 }
 template <class F>
 __device__ __forceinline__ float sample(const F& f, float gx, float gy, float ox, float oy) {
-  const float fxp = gx - ox, fyp = gy - oy;
-  const float bx = floorf(fxp), by = floorf(fyp), tx = fxp - bx, ty = fyp - by;
-  const int i = wgsl_i32(bx), j = wgsl_i32(by);
+  float tx, ty;
+  const int i = floor_frac(gx - ox, tx), j = floor_frac(gy - oy, ty);
   float A, C, D, E;
   corners(f, i, j, A, C, D, E);
   return mixf(mixf(A, C, tx), mixf(D, E, tx), ty);
 }
 template <class F>
 __device__ __forceinline__ float4 sample4(const F& f, float gx, float gy) {
-  const float fxp = gx - 0.5f, fyp = gy - 0.5f;
-  const float bx = floorf(fxp), by = floorf(fyp), tx = fxp - bx, ty = fyp - by;
-  const int i = wgsl_i32(bx), j = wgsl_i32(by);
+  float tx, ty;
+  const int i = floor_frac(gx - 0.5f, tx), j = floor_frac(gy - 0.5f, ty);
   float4 A, C, D, E;
   corners(f, i, j, A, C, D, E);
   return mix4(mix4(A, C, tx), mix4(D, E, tx), ty);
 }
-// mm_<name>: min/max of the 4 corners
-template <class F>
-__device__ __forceinline__ void minmax(const F& f, float gx, float gy, float ox, float oy, float& lo, float& hi) {
-  const int i = wgsl_i32(floorf(gx - ox)), j = wgsl_i32(floorf(gy - oy));
-  float A, C, D, E;
-  corners(f, i, j, A, C, D, E);
-  lo = fminf(fminf(A, C), fminf(D, E)); hi = fmaxf(fmaxf(A, C), fmaxf(D, E));
-}
-template <class F>
-__device__ __forceinline__ void minmax4(const F& f, float gx, float gy, float4& lo, float4& hi) {
-  const int i = wgsl_i32(floorf(gx - 0.5f)), j = wgsl_i32(floorf(gy - 0.5f));
-  float4 A, C, D, E;
-  corners(f, i, j, A, C, D, E);
-  lo = min4(min4(A, C), min4(D, E)); hi = max4(max4(A, C), max4(D, E));
-}
-
 // x / d rounded to nearest from r = RN(1/d): q0 = RN(x r), q = RN(q0 + r (x - d q0)),
 // the residual x - d q0 exact by FMA (Markstein, IBM J. Res. Dev. 34(1), 1990). Equal
 // to the IEEE quotient for quotients in the normal range (and for x = +0); for x = -0 it

@@ -9,7 +9,7 @@ namespace cfg {
 // Tile shapes (cells) of the level-0 kernels. Tiles are aligned to multiples of
 // 8 cells so the 8x8 blocks of the heat-release reduction match the WGSL
 // workgroups of sources.wgsl:34 exactly.
-constexpr int ADV_TX = 32, ADV_TY = 8, ADV_H = 2;    // advection (halo for |displacement| < 2 cells)
+constexpr int ADV_TX = 32, ADV_TY = 8, ADV_H = 4;    // advection (widest halo staged: displacements under 4 cells)
 constexpr int DS_TX = 32, DS_TY = 8;                 // diffusion + sources
 constexpr int FR_TX = 32, FR_TY = 8;                 // forces + coef + rhs0 (+ coefficient hierarchy)
 // Tile shapes the advection, diffusion + sources and forces kernels can run with (the
