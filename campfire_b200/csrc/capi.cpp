@@ -258,6 +258,7 @@ extern "C" int cfg_autotune(int device, int nscenes, const int* nx, const int* n
   return guarded([&] {
     std::vector<double> width(nscenes, 0.8), dt(nscenes, 0.002);
     cfg::Engine eng;
+    eng.uncap_block();
     CFG_TRY(eng.init(device, nscenes, nx, ny, width.data(), dt.data()));
     for (int s = 0; s < nscenes; s++) CFG_TRY(cfg::load_generated_scene(eng, s, 0, 0.8, 1234 + s));
     if (coarse_direct) {

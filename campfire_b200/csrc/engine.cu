@@ -118,10 +118,15 @@ int Engine::activate() const {
 }
 
 // The coarse block starts at the first level with at most `cells` cells whose
-// arrays fit in one CTA's shared memory (else at the coarsest level).
+// arrays fit in one CTA's shared memory (else at the coarsest level), or later: `cap` cells at
+// most (level 0, which a block may cover whole, only where `cap0`). Every start gives the same
+// pressures; above kBlockCells the tiled kernels of a level are the faster ones, ~7 us down and
+// up against 12-17 us on one SM (per step: 128x192 in FP32 cycles 344 -> 268 us with 64x96 tiled,
+// 224x320 126 -> 113 with 56x80 tiled; 1536 to 4600 cells differ by under 2%). In the FP64
+// modes a block that covers level 0 stays: the loop's update follows from it.
 // cs > 0: the cluster coarse phase, which starts at level 1 at the earliest (level 0
 // always runs as tiled kernels) and fits each CTA's share of the levels
-int Engine::choose_lc(const Scene& sc, int cells, int cs) {
+int Engine::choose_lc(const Scene& sc, int cells, int cs, int cap, bool cap0) {
   if (cs > 0) {
     for (int l = std::min(1, sc.nlev - 1); l < sc.nlev; l++)
       if (sc.lnx[l] * sc.lny[l] <= cells && cluster_smem_bytes(sc.lnx, sc.lny, l, sc.nlev, cs) <= kClusterSmemMax)
@@ -129,7 +134,11 @@ int Engine::choose_lc(const Scene& sc, int cells, int cs) {
     return sc.nlev - 1;
   }
   for (int l = 0; l < sc.nlev; l++)
-    if (sc.lnx[l] * sc.lny[l] <= cells && coarse_smem_bytes(sc.lnx, sc.lny, l, sc.nlev) <= kCoarseSmemMax) return l;
+    if (sc.lnx[l] * sc.lny[l] <= cells && coarse_smem_bytes(sc.lnx, sc.lny, l, sc.nlev) <= kCoarseSmemMax) {
+      if (l > 0 || cap0)
+        while (l + 1 < sc.nlev && sc.lnx[l] * sc.lny[l] > cap) l++;
+      return l;
+    }
   return sc.nlev - 1;
 }
 
@@ -152,7 +161,7 @@ int Engine::init(int device, int n, const int* nx, const int* ny, const double* 
     }
     sc.nlev = L;
     if (sc.lnx[L - 1] * sc.lny[L - 1] > 256) return fail(CFG_ERR_RANGE, "coarsest level too large");
-    sc.lc = choose_lc(sc, coarse_cells_, 0);
+    sc.lc = choose_lc(sc, coarse_cells_, 0, block_cap_, true);
     coarse_smem_ = std::max(coarse_smem_, coarse_smem_bytes(sc.lnx, sc.lny, sc.lc, sc.nlev));
     const int cn = sc.lnx[L - 1] * sc.lny[L - 1], cbw = sc.lnx[L - 1];
     if (cbw <= 32) { cf_smem_ = std::max(cf_smem_, coarse_factor_smem(cn, cbw)); cf_bw_ = std::max(cf_bw_, cbw); }
@@ -521,7 +530,8 @@ int Engine::set_coarse_cells(int cells) {
     int lw = MAX_LEVELS;
     if (w_cells_ > 0 && sc.nlev >= 3 && sc.lnx[sc.nlev - 3] * sc.lny[sc.nlev - 3] <= w_cells_) lw = sc.nlev - 3;
     lws[s] = lw;
-    lcs[s] = choose_lc(sc, std::max(cells, lw < sc.nlev ? sc.lnx[lw] * sc.lny[lw] : 0), cs);
+    const int lwc = lw < sc.nlev ? sc.lnx[lw] * sc.lny[lw] : 0;
+    lcs[s] = choose_lc(sc, std::max(cells, lwc), cs, std::max(block_cap_, lwc), !any_fp64());
     if (lw < sc.nlev && lcs[s] > lw)
       return fail(CFG_ERR_RANGE, "the W tail's levels do not fit in the coarse block's shared memory");
     smem = std::max(smem, cs > 0 ? cluster_smem_bytes(sc.lnx, sc.lny, lcs[s], sc.nlev, cs)
@@ -1144,8 +1154,13 @@ int Engine::set_solver(int mode, int ncycles, double tol, int max_cycles) {
   if (mode == CFG_SOLVE_FIXED && ncycles < 1) return fail(CFG_ERR_INVAL, "ncycles must be >= 1");
   if (mode != CFG_SOLVE_FIXED && (!(tol > 0) || max_cycles < 1)) return fail(CFG_ERR_INVAL, "tol must be > 0 and max_cycles >= 1");
   CFG_TRY(activate());
+  const bool was = any_fp64();
   mode_ = mode; ncycles_ = ncycles; tol_ = tol; max_cycles_ = max_cycles;
   graph_dirty_ = true;
+  // a block that may cover level 0 in one kind of mode only
+  if (any_fp64() != was && coarse_cluster_ == 0)
+    for (const Scene& sc : scenes_)
+      if (sc.nx * sc.ny > block_cap_ && sc.nx * sc.ny <= coarse_cells_) { CFG_TRY(set_coarse_cells(coarse_cells_)); break; }
   return upload_ctl();
 }
 
@@ -1158,8 +1173,6 @@ void Engine::enqueue_pre_solve(cudaStream_t s, unsigned long long h, int use_con
   if (FR_KMAX + 1 < max_levels()) { launch_coef_restrict_tail(d_scenes_, nscenes(), FR_KMAX, s); launches_++; }
   enqueue_factor(s);
   if (fp64) { launch_defect64(d_scenes_, nscenes(), d_wl_[WL_MG0], nwl_[WL_MG0], d_ctl_, 1, s); launches_++; }
-  // the loop's cycle counter starts at zero in every step
-  cudaMemsetAsync(&d_ctl_->iter, 0, sizeof(int), s);
   (void)h; (void)use_cond;
 }
 
@@ -1230,18 +1243,23 @@ void Engine::enqueue_loop_end(cudaStream_t s) {
 // The step's V(2,2) cycle with the fused kernels (k_mgf.cu); the level-0 up
 // kernel (or the coarse block of scenes whose block starts at level 0) ends
 // the cycle with the residual norm (FP32 modes) or p64 += p (FP64 mode).
-void Engine::enqueue_vcycle(cudaStream_t s, int tail, int count_iter) {
+// pdl_first: whether the first kernel may be launched before its predecessor has completed (in the
+// loop's body; not straight after the kernels that build the coefficients, which the smoothers
+// read before their wait)
+void Engine::enqueue_vcycle(cudaStream_t s, int tail, int count_iter, bool pdl_first) {
   const int LD = max_lc();
+  bool pdl = pdl_first;
   for (int l = 0; l < LD; l++) {
     if (nwl_[WL_MGD0 + l] == 0) continue;
-    launch_mg_down(d_scenes_, nscenes(), d_wl_[WL_MGD0 + l], nwl_[WL_MGD0 + l], l, d_ctl_, count_iter, tail == 4 && l == 0, s);
+    launch_mg_down(d_scenes_, nscenes(), d_wl_[WL_MGD0 + l], nwl_[WL_MGD0 + l], l, d_ctl_, count_iter, tail == 4 && l == 0, pdl, s);
     count_iter = 0;
+    pdl = true;
     vcycle_launches_++;
   }
   if (coarse_cluster_ > 0)
     launch_mg_cluster(d_scenes_, nscenes(), d_ctl_, coarse_cluster_, count_iter, cluster_smem_, s);
   else
-    launch_mg_coarse(d_scenes_, nscenes(), d_ctl_, tail, count_iter, coarse_smem_, any_wtail(), any_block_level0(), s);
+    launch_mg_coarse(d_scenes_, nscenes(), d_ctl_, tail, count_iter, coarse_smem_, any_wtail(), any_block_level0(), pdl, s);
   vcycle_launches_++;
   for (int l = LD - 1; l >= 0; l--) {
     if (nwl_[WL_MGD0 + l] == 0) continue;
@@ -1403,33 +1421,43 @@ int Engine::ensure_graph() {
   };
   cudaError_t e = cudaStreamGetCaptureInfo(s, &status, nullptr, &g, nullptr, nullptr);
   if (e != cudaSuccess) return abort_capture(e, "cudaStreamGetCaptureInfo");
+  // A few cycles of a fixed count are laid out one after the other: there is nothing to decide, and
+  // the loop node cost a step of one cycle 16 us (224x320: 113 -> 96 us). Longer and undecided loops are a WHILE node.
+  const bool unrolled = mode_ == CFG_SOLVE_FIXED && ncycles_ <= kUnrolledCycles && coarse_cluster_ == 0;
   cudaGraphConditionalHandle h = 0;
-  e = cudaGraphConditionalHandleCreate(&h, g, 1, cudaGraphCondAssignDefault);
-  if (e != cudaSuccess) return abort_capture(e, "cudaGraphConditionalHandleCreate");
   launches_ = 0;
-  enqueue_pre_solve(s, (unsigned long long)h, 1);
-  e = cudaStreamGetCaptureInfo(s, &status, nullptr, &g, &deps, &ndeps);
-  if (e != cudaSuccess) return abort_capture(e, "cudaStreamGetCaptureInfo");
-  cudaGraphNodeParams cp = {};
-  cp.type = cudaGraphNodeTypeConditional;
-  cp.conditional.handle = h;
-  cp.conditional.type = cudaGraphCondTypeWhile;
-  cp.conditional.size = 1;
-  cudaGraphNode_t cnode;
-  e = cudaGraphAddNode(&cnode, g, deps, ndeps, &cp);
-  if (e != cudaSuccess) return abort_capture(e, "cudaGraphAddNode(while)");
-  cudaGraph_t body = cp.conditional.phGraph_out[0];
-  e = cudaStreamUpdateCaptureDependencies(s, &cnode, 1, cudaStreamSetCaptureDependencies);
-  if (e != cudaSuccess) return abort_capture(e, "cudaStreamUpdateCaptureDependencies");
-  e = cudaStreamBeginCaptureToGraph(body_stream_, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
-  if (e != cudaSuccess) return abort_capture(e, "cudaStreamBeginCaptureToGraph");
-  vcycle_launches_ = 0;
-  // the first kernel of the body counts the iteration and the cycle's decision sets the
-  // condition (loop_count / solve_decide): no guard kernel in the body
-  enqueue_vcycle(body_stream_, cycle_tail(), 1);
-  enqueue_fp64_tail(body_stream_);
-  e = cudaStreamEndCapture(body_stream_, &body);
-  if (e != cudaSuccess) return abort_capture(e, "cudaStreamEndCapture(body)");
+  if (unrolled) {
+    enqueue_pre_solve(s, 0ull, 0);
+    vcycle_launches_ = 0;
+    for (int k = 0; k < ncycles_; k++) enqueue_vcycle(s, cycle_tail(), 0, k > 0);
+    vcycle_launches_ /= ncycles_;
+  } else {
+    e = cudaGraphConditionalHandleCreate(&h, g, 1, cudaGraphCondAssignDefault);
+    if (e != cudaSuccess) return abort_capture(e, "cudaGraphConditionalHandleCreate");
+    enqueue_pre_solve(s, (unsigned long long)h, 1);
+    e = cudaStreamGetCaptureInfo(s, &status, nullptr, &g, &deps, &ndeps);
+    if (e != cudaSuccess) return abort_capture(e, "cudaStreamGetCaptureInfo");
+    cudaGraphNodeParams cp = {};
+    cp.type = cudaGraphNodeTypeConditional;
+    cp.conditional.handle = h;
+    cp.conditional.type = cudaGraphCondTypeWhile;
+    cp.conditional.size = 1;
+    cudaGraphNode_t cnode;
+    e = cudaGraphAddNode(&cnode, g, deps, ndeps, &cp);
+    if (e != cudaSuccess) return abort_capture(e, "cudaGraphAddNode(while)");
+    cudaGraph_t body = cp.conditional.phGraph_out[0];
+    e = cudaStreamUpdateCaptureDependencies(s, &cnode, 1, cudaStreamSetCaptureDependencies);
+    if (e != cudaSuccess) return abort_capture(e, "cudaStreamUpdateCaptureDependencies");
+    e = cudaStreamBeginCaptureToGraph(body_stream_, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
+    if (e != cudaSuccess) return abort_capture(e, "cudaStreamBeginCaptureToGraph");
+    vcycle_launches_ = 0;
+    // the first kernel of the body counts the iteration and the cycle's decision sets the
+    // condition (loop_count / solve_decide): no guard kernel in the body
+    enqueue_vcycle(body_stream_, cycle_tail(), 1);
+    enqueue_fp64_tail(body_stream_);
+    e = cudaStreamEndCapture(body_stream_, &body);
+    if (e != cudaSuccess) return abort_capture(e, "cudaStreamEndCapture(body)");
+  }
   enqueue_loop_end(s);
   e = enqueue_post_solve(s);
   if (e != cudaSuccess) return abort_capture(e, "enqueue_post_solve");
@@ -1439,6 +1467,7 @@ int Engine::ensure_graph() {
   e = cudaGraphInstantiate(&exec_, graph_, 0);
   if (e != cudaSuccess) { destroy_graph(); return cuda_fail(e, "cudaGraphInstantiate"); }
   cond_handle_ = (unsigned long long)h;
+  graph_loops_ = !unrolled;
   ctl_use_cond_ = -1;   // upload the new handle before the next launch
   graph_dirty_ = false;
   graph_sub_ = max_sub();
@@ -1458,7 +1487,7 @@ int Engine::step(int nsteps) {
         graph_dirty_ = true;
         CFG_TRY(ensure_graph());
       }
-      CFG_TRY(set_cond_mode(true));
+      CFG_TRY(set_cond_mode(graph_loops_));
       CFG_CUDA(cudaGraphLaunch(exec_, st()));
       dt_from_step_ = dt_from_step_ || any_cfl();
       mark_device_dt();
@@ -1603,7 +1632,7 @@ int Engine::time_kernel(const char* name, int iters, double* ms, double* bytes, 
     go = [&](int) { launch_coarsest(d_scenes_, nscenes(), s); };
     b = 0; cnt = cyc;
   } else if (n == "mg_down0") {
-    go = [&](int) { launch_mg_down(d_scenes_, nscenes(), d_wl_[WL_MGD0], nwl_[WL_MGD0], 0, d_ctl_, 0, 0, s); };
+    go = [&](int) { launch_mg_down(d_scenes_, nscenes(), d_wl_[WL_MGD0], nwl_[WL_MGD0], 0, d_ctl_, 0, 0, true, s); };
     b = (4 * 16 + 18) * cells; cnt = cyc;   // 4 colour passes + residual restriction
   } else if (n == "mg_up0") {
     go = [&](int) { launch_mg_up(d_scenes_, nscenes(), d_wl_[WL_MGD0], nwl_[WL_MGD0], 0, 0, d_ctl_, s); };
@@ -1613,7 +1642,7 @@ int Engine::time_kernel(const char* name, int iters, double* ms, double* bytes, 
     // the V-cycle's bytes plus half of the FP64 iteration's 40 B per cell each
     if (!pcg_fused()) return fail(CFG_ERR_NOENT, n + ": the Krylov update is not folded in this engine");
     if (n == "mg_down0_krylov") {
-      go = [&](int) { launch_mg_down(d_scenes_, nscenes(), d_wl_[WL_MGD0], nwl_[WL_MGD0], 0, d_ctl_, 0, 1, s); };
+      go = [&](int) { launch_mg_down(d_scenes_, nscenes(), d_wl_[WL_MGD0], nwl_[WL_MGD0], 0, d_ctl_, 0, 1, true, s); };
       b = (4 * 16 + 18 + 20) * cells;
     } else {
       go = [&](int) { launch_mg_up(d_scenes_, nscenes(), d_wl_[WL_MGD0], nwl_[WL_MGD0], 0, 4, d_ctl_, s); };
@@ -1631,7 +1660,7 @@ int Engine::time_kernel(const char* name, int iters, double* ms, double* bytes, 
   } else if (n == "mg_coarse") {
     go = [&](int) {
       if (coarse_cluster_ > 0) launch_mg_cluster(d_scenes_, nscenes(), d_ctl_, coarse_cluster_, 0, cluster_smem_, s);
-      else launch_mg_coarse(d_scenes_, nscenes(), d_ctl_, 0, 0, coarse_smem_, any_wtail(), any_block_level0(), s);
+      else launch_mg_coarse(d_scenes_, nscenes(), d_ctl_, 0, 0, coarse_smem_, any_wtail(), any_block_level0(), true, s);
     };
     // the reference schedule's V-cycle bytes of the levels the block covers (163 B per level cell)
     b = 0;
@@ -1661,7 +1690,7 @@ int Engine::time_kernel(const char* name, int iters, double* ms, double* bytes, 
   } else if (n.size() == 8 && (n.compare(0, 7, "mg_down") == 0) && n[7] >= '1' && n[7] <= '6') {
     const int l = n[7] - '0';
     if (l >= sc.lc) return fail(CFG_ERR_NOENT, "level " + n.substr(7) + " is in the coarse block");
-    go = [&, l](int) { launch_mg_down(d_scenes_, nscenes(), d_wl_[WL_MGD0 + l], nwl_[WL_MGD0 + l], l, d_ctl_, 0, 0, s); };
+    go = [&, l](int) { launch_mg_down(d_scenes_, nscenes(), d_wl_[WL_MGD0 + l], nwl_[WL_MGD0 + l], l, d_ctl_, 0, 0, true, s); };
     b = (4 * 16 + 18) * (double)sc.lnx[l] * sc.lny[l]; cnt = cyc;
   } else if (n.size() == 6 && (n.compare(0, 5, "mg_up") == 0) && n[5] >= '1' && n[5] <= '6') {
     const int l = n[5] - '0';

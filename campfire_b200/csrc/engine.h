@@ -163,6 +163,7 @@ class Engine {
   // most `cells` cells (levels above it run as tiled down/up kernels)
   int set_coarse_cells(int cells);
   int coarse_cells() const { return coarse_cells_; }
+  void uncap_block() { block_cap_ = 1 << 30; }   // the autotuner times every start as asked
   // cycle shape of the pressure loop: with cells > 0, the level two above the coarsest visits
   // its coarser level twice per cycle (the W tail) when it has at most `cells` cells; that
   // level always runs inside the one-CTA coarse block
@@ -196,7 +197,7 @@ class Engine {
   int nscenes() const { return (int)scenes_.size(); }
 
  private:
-  static int choose_lc(const Scene& sc, int cells, int cs);
+  static int choose_lc(const Scene& sc, int cells, int cs, int cap, bool cap0);
   int alloc_scene(Scene& sc);
   int build_tmaps(Scene& sc);
   int upload_desc(int s);
@@ -215,7 +216,7 @@ class Engine {
   // step pieces; launches counted in launches_
   void enqueue_pre_solve(cudaStream_t s, unsigned long long h, int use_cond);
   // fused kernels (the step's cycle); tail as k_mg_up; count_iter: the first kernel opens a graph iteration
-  void enqueue_vcycle(cudaStream_t s, int tail, int count_iter);
+  void enqueue_vcycle(cudaStream_t s, int tail, int count_iter, bool pdl_first = true);
   void enqueue_vcycle_ref(cudaStream_t s);   // one kernel per reference dispatch (cfg_vcycle)
   int max_lc() const;
   bool direct_coarse() const { return mode_ != CFG_SOLVE_FIXED && coarse_direct_ != 0; }
@@ -276,6 +277,8 @@ class Engine {
   size_t cluster_smem_ = 0;
   int cf_bw_ = 0;               // the widest coarsest level (k_coarse_factor's register window)
   int coarse_cells_ = COARSE_CELLS;
+  int block_cap_ = kBlockCells;
+  bool graph_loops_ = true;   // the step graph holds the pressure loop's WHILE node
   int w_cells_ = 0;             // set_coarse_w
   int coarse_direct_ = 0;
   int krylov_ = 0;

@@ -209,6 +209,7 @@ __global__ void __launch_bounds__(256) k_forces(const SceneDesc* __restrict__ sc
       ctl->scenes_done = 0u;
       ctl->nactive = ctl->nscenes;
       ctl->any_active = 1;
+      ctl->iter = 0;   // the loop's cycle counter
     }
   }
 }

@@ -1395,14 +1395,14 @@ static bool one_wave_at_two(int ntiles) {
   return ntiles <= 2 * sms;
 }
 void launch_mg_down(const SceneDesc* scenes, int nscenes, const Work* work, int ntiles, int level, SolveCtl* ctl,
-                    int count_iter, int pcg, cudaStream_t st) {
+                    int count_iter, int pcg, bool pdl, cudaStream_t st) {
   if (ntiles <= 0) return;
   const auto k = nscenes == 1
                      ? (pcg ? (one_wave_at_two(ntiles) ? k_mg_down<MGF_TX, MGF_TY, true, true, 2>
                                                        : k_mg_down<MGF_TX, MGF_TY, true, true>)
                             : k_mg_down<MGF_TX, MGF_TY, false, true>)
                      : (pcg ? k_mg_down<MGF_TX, MGF_TY, true, false> : k_mg_down<MGF_TX, MGF_TY, false, false>);
-  launch_pdl(pdl_enabled(), k, dim3(ntiles), dim3(256), 0, st, scenes, nscenes, work, level, ctl, count_iter);
+  launch_pdl(pdl && pdl_enabled(), k, dim3(ntiles), dim3(256), 0, st, scenes, nscenes, work, level, ctl, count_iter);
 }
 void launch_mg_up(const SceneDesc* scenes, int nscenes, const Work* work, int ntiles, int level, int tail, SolveCtl* ctl,
                   cudaStream_t st) {
@@ -1416,9 +1416,9 @@ void launch_pcg_decide(const SceneDesc* scenes, int nscenes, SolveCtl* ctl, cuda
   if (nscenes > 0) launch_pdl(pdl_enabled(), k_pcg_decide, dim3(nscenes), dim3(256), 0, st, scenes, ctl);
 }
 void launch_mg_coarse(const SceneDesc* scenes, int nscenes, SolveCtl* ctl, int tail, int count_iter, size_t smem,
-                      int wtail, int level0, cudaStream_t st) {
+                      int wtail, int level0, bool pdl, cudaStream_t st) {
   if (nscenes > 0)
-    launch_pdl(pdl_enabled(),
+    launch_pdl(pdl && pdl_enabled(),
                wtail ? (level0 ? k_mg_coarse<true, true> : k_mg_coarse<true, false>)
                      : (level0 ? k_mg_coarse<false, true> : k_mg_coarse<false, false>),
                dim3(nscenes), dim3(CB_THREADS), smem, st, scenes, nscenes, ctl, tail, count_iter, (int)(smem / 4));

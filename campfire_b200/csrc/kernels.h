@@ -35,6 +35,8 @@ constexpr int MGF_CBW = MGF_TX / 2 + 16, MGF_CBH = MGF_TY / 2 + 8;        // coa
 enum TmapKind { TM_P = 0, TM_PB, TM_RHS, TM_AX, TM_AY, TM_PC, TM_PER_LEVEL };
 constexpr int TMAP_BYTES = 128;
 constexpr int COARSE_CELLS = 6144;                   // default: largest level handled by the one-CTA coarse block
+constexpr int kBlockCells = 2048;                    // the block starts no earlier than a level of this size (Engine::choose_lc)
+constexpr int kUnrolledCycles = 4;                   // fixed cycle counts up to this many are unrolled in the step graph
 constexpr size_t kCoarseSmemMax = 232448 - 2048;     // dynamic shared memory of the coarse block (227 KB less static)
 constexpr int PR_TX = 32, PR_TY = 8;                 // projection
 static_assert(PR_TX == MG_TX && PR_TY == MG_TY, "the projection's tiles are counted as the level-0 multigrid tiles");
@@ -110,7 +112,7 @@ void launch_readback(uint32_t* src, uint32_t* host, int nwords, int nzero, cudaS
 // fused Krylov mode (applies the previous cycle's update); nscenes: the engine's scenes
 // (with one, tiles are requested before the scene's active flag is read: it only stops the loop)
 void launch_mg_down(const SceneDesc* scenes, int nscenes, const Work* work, int ntiles, int level, SolveCtl* ctl,
-                    int count_iter, int pcg, cudaStream_t st);
+                    int count_iter, int pcg, bool pdl, cudaStream_t st);
 void launch_mg_up(const SceneDesc* scenes, int nscenes, const Work* work, int ntiles, int level, int tail, SolveCtl* ctl,
                   cudaStream_t st);
 // after the level-0 up kernel with tail 4: each scene's dot products summed, the coefficients
@@ -120,7 +122,7 @@ void launch_pcg_decide(const SceneDesc* scenes, int nscenes, SolveCtl* ctl, cuda
 // scene's block covers level 0 (the cycle's level-0 ends: warm start, `tail`), else an instance
 // without them
 void launch_mg_coarse(const SceneDesc* scenes, int nscenes, SolveCtl* ctl, int tail, int count_iter, size_t smem,
-                      int wtail, int level0, cudaStream_t st);
+                      int wtail, int level0, bool pdl, cudaStream_t st);
 size_t coarse_smem_bytes(const int* lnx, const int* lny, int lc, int nlev);
 // the cluster coarse phase (k_mgc.cu): levels lc..coarsest of each scene on a cluster of cs CTAs
 constexpr size_t kClusterSmemMax = 232448 - 2048;

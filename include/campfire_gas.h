@@ -203,7 +203,9 @@ int cfg_time_kernel(cfg_sim* sim, const char* kernel, int iters, double* mean_ms
 /* Smoother schedule (no counterpart in the reference, whose schedule is fixed): the levels
  * from the first one with at most `cells` cells down to the coarsest run in one CTA per
  * scene, the levels above as tiled down/up kernels. Results are bit-identical for every
- * choice; only the time changes. Default 6144. Batch views: use cfg_batch_set_coarse_cells. */
+ * choice; only the time changes, and levels above 2048 cells, on which the tiled kernels are
+ * faster, run tiled whatever the choice (in the FP64 modes a block that covers level 0 stays
+ * whole). Default 6144. Batch views: use cfg_batch_set_coarse_cells. */
 int cfg_set_coarse_cells(cfg_sim* sim, int cells);
 /* Where that coarse phase runs: 0 (default) one CTA per scene; 2, 4, 8 or 16: a thread-block
  * cluster of that many CTAs per scene, each owning a share of every level's rows (from level 1
