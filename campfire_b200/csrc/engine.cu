@@ -1421,20 +1421,33 @@ int Engine::ensure_graph() {
   };
   cudaError_t e = cudaStreamGetCaptureInfo(s, &status, nullptr, &g, nullptr, nullptr);
   if (e != cudaSuccess) return abort_capture(e, "cudaStreamGetCaptureInfo");
-  // A few cycles of a fixed count are laid out one after the other: there is nothing to decide, and
-  // the loop node cost a step of one cycle 16 us (224x320: 113 -> 96 us). Longer and undecided loops are a WHILE node.
-  const bool unrolled = mode_ == CFG_SOLVE_FIXED && ncycles_ <= kUnrolledCycles && coarse_cluster_ == 0;
+  // The first cycles are laid out one after the other, up to kUnrolledCycles: all of a fixed count, or
+  // one per decade of the asked tolerance (what the solves need or a little less: 5-6 for 1e-6,
+  // 9-11 for 1e-10). Only what remains is a WHILE node, which costs a step ~10 us to enter and 5 us
+  // between two cycles (256x384: 48 us per looped cycle, 43 per laid-out one) where a laid-out cycle
+  // after the last needed one costs 8 us (512x768: 13), its kernels leaving on the scene's flag.
+  const bool fixed = mode_ == CFG_SOLVE_FIXED;
+  const int wanted = fixed ? ncycles_ : (int)std::lround(-std::log10(tol_));
+  const int ahead = coarse_cluster_ > 0 ? 0 : std::min(std::max(std::min(wanted, fixed ? ncycles_ : max_cycles_), 0), kUnrolledCycles);
+  const bool unrolled = fixed && ahead == ncycles_;   // nothing to decide, no loop
   cudaGraphConditionalHandle h = 0;
   launches_ = 0;
-  if (unrolled) {
-    enqueue_pre_solve(s, 0ull, 0);
-    vcycle_launches_ = 0;
-    for (int k = 0; k < ncycles_; k++) enqueue_vcycle(s, cycle_tail(), 0, k > 0);
-    vcycle_launches_ /= ncycles_;
-  } else {
+  if (!unrolled) {
     e = cudaGraphConditionalHandleCreate(&h, g, 1, cudaGraphCondAssignDefault);
     if (e != cudaSuccess) return abort_capture(e, "cudaGraphConditionalHandleCreate");
-    enqueue_pre_solve(s, (unsigned long long)h, 1);
+  }
+  enqueue_pre_solve(s, (unsigned long long)h, unrolled ? 0 : 1);
+  // the first kernel of every cycle counts it and the cycle's decision sets the loop's condition
+  // (loop_count / solve_decide): no guard kernel
+  vcycle_launches_ = 0;
+  for (int k = 0; k < ahead; k++) {
+    enqueue_vcycle(s, cycle_tail(), 1, k > 0);
+    enqueue_fp64_tail(s);
+  }
+  if (unrolled) {
+    vcycle_launches_ /= ahead;
+  } else {
+    vcycle_launches_ = 0;
     e = cudaStreamGetCaptureInfo(s, &status, nullptr, &g, &deps, &ndeps);
     if (e != cudaSuccess) return abort_capture(e, "cudaStreamGetCaptureInfo");
     cudaGraphNodeParams cp = {};
@@ -1450,9 +1463,6 @@ int Engine::ensure_graph() {
     if (e != cudaSuccess) return abort_capture(e, "cudaStreamUpdateCaptureDependencies");
     e = cudaStreamBeginCaptureToGraph(body_stream_, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) return abort_capture(e, "cudaStreamBeginCaptureToGraph");
-    vcycle_launches_ = 0;
-    // the first kernel of the body counts the iteration and the cycle's decision sets the
-    // condition (loop_count / solve_decide): no guard kernel in the body
     enqueue_vcycle(body_stream_, cycle_tail(), 1);
     enqueue_fp64_tail(body_stream_);
     e = cudaStreamEndCapture(body_stream_, &body);

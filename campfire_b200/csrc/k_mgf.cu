@@ -82,6 +82,13 @@ __device__ __forceinline__ const void* tmap_of(const SceneDesc& S, int level, in
   return S.tmap + (size_t)(level * TM_PER_LEVEL + kind) * TMAP_BYTES;
 }
 
+// Whether the scene has stopped cycling, asked before the wait on the previous kernel: the flag
+// only falls during a loop (the kernels before the loop raise it, and no loop kernel starts
+// before they have completed), so a zero stands whatever the previous kernel still does. A one
+// may be stale; the flag is read again after the wait. A laid-out cycle after the last one
+// needed then costs its kernels' launches only.
+__device__ __forceinline__ bool scene_idle(const SolveState* ss) { return *(const volatile int*)&ss->active == 0; }
+
 // Tile staging on two barriers around the wait on the previous kernel. stage_coef
 // (before the wait in a one-scene engine, which also waits for them and builds the stencils
 // before the wait, with the state copies' tensor maps prefetched; else once the scene's flag
@@ -380,9 +387,14 @@ __global__ void __launch_bounds__(256, MINB) k_mg_down(const SceneDesc* __restri
   // one scene: its flag only ends the loop, so the tile is requested before it is read;
   // several: a scene that stopped loads nothing
   constexpr bool spec = ONE;
-  if (on && spec) {
-    stage_coef(S, level, t, bar);
-    prefetch_state_maps(S, level, TM_P, false);
+  __shared__ int s_idle;   // thread 0's reading: the flag may fall while the CTA's threads would read it
+  if (on && spec && threadIdx.x == 0) {
+    const bool z = scene_idle(ss);
+    s_idle = z;
+    if (!z) {
+      stage_coef(S, level, t, bar);
+      prefetch_state_maps(S, level, TM_P, false);
+    }
   }
   // below level 0 the level's p is zero on entry (the restriction above zeroes it): with one
   // scene its box is zero-filled before the wait instead of copied after it
@@ -390,13 +402,14 @@ __global__ void __launch_bounds__(256, MINB) k_mg_down(const SceneDesc* __restri
   if (pz)
     for (int e = threadIdx.x; e < MGF_BW * MGF_BH; e += 256) t.p[e] = 0.f;
   __syncthreads();
+  const bool idle = on && spec && s_idle;
   // one scene: the stencils, which depend on the coefficients alone, are built before the wait
   TCell c[2][2];
   bool ok = true;
-  if (on && spec && (ok = tile_wait(&bar[0], ctl))) tile_stencils(t, L, x0, y0, 0, c);
+  if (on && spec && !idle && (ok = tile_wait(&bar[0], ctl))) tile_stencils(t, L, x0, y0, 0, c);
   pdl_wait();
   if (count_iter && blockIdx.x == 0 && threadIdx.x == 0) loop_count(ctl);
-  if (!on || !ok) return;
+  if (!on || !ok || idle) return;
   if (!spec) {
     if (*(volatile int*)&ss->active == 0) return;
     stage_coef(S, level, t, bar);
@@ -484,23 +497,29 @@ __global__ void __launch_bounds__(256, MINB) k_mg_up(const SceneDesc* __restrict
   const bool on = S.enabled;   // host-written, constant during the step
   SolveState* ss = S.solve;
   constexpr bool spec = ONE;   // as in k_mg_down
-  if (on && spec) {
-    stage_coef(S, level, t, bar);
-    prefetch_state_maps(S, level, TM_PB, true);
+  __shared__ int s_idle;
+  if (on && spec && threadIdx.x == 0) {
+    const bool z = scene_idle(ss);
+    s_idle = z;
+    if (!z) {
+      stage_coef(S, level, t, bar);
+      prefetch_state_maps(S, level, TM_PB, true);
+    }
   }
   __shared__ double s_rh2;   // the FP64 operator's 1 / h2 (tails 3 and 4)
   if (threadIdx.x == 0) s_rh2 = 1.0 / (double)L.h2;
   __syncthreads();
+  const bool idle = on && spec && s_idle;
   const double rh2 = s_rh2;
   TCell c[2][2];
   uint32_t pl[PR_N];
   bool ok = true;
-  if (on && spec && (ok = tile_wait(&bar[0], ctl))) {
+  if (on && spec && !idle && (ok = tile_wait(&bar[0], ctl))) {
     tile_stencils(t, L, x0, y0, 1, c);
     prolong_plan(t, L, C, x0, y0, cx, cy, pl);
   }
   pdl_wait();
-  if (!on || !ok) return;
+  if (!on || !ok || idle) return;
   if (!spec) {
     if (*(volatile int*)&ss->active == 0) return;
     stage_coef(S, level, t, bar);
@@ -1017,6 +1036,7 @@ __global__ void __launch_bounds__(CB_THREADS) k_mg_coarse(const SceneDesc* __res
   __shared__ double red[32];
   __shared__ LvO lvo[MAX_LEVELS];
   __shared__ __align__(8) uint64_t bar;    // the coefficients (+ inverse)
+  __shared__ int s_idle;                          // as in k_mg_down
   __shared__ int s_inv, s_res, s_A, s_dir, s_gpc;   // offsets: residual scratch, inverse
   __shared__ float* s_gp;                         // level lc's p in global memory
   const SceneDesc& S = scenes[blockIdx.x];
@@ -1043,6 +1063,7 @@ __global__ void __launch_bounds__(CB_THREADS) k_mg_coarse(const SceneDesc* __res
     q = round_up(q, 32);
     s_A = q;
     s_gp = S.lev[lc].p; s_gpc = S.lev[lc].pc;
+    s_idle = scene_idle(S.solve);
     mbar_init(&bar, 1);
   }
   __syncthreads();
@@ -1054,8 +1075,8 @@ __global__ void __launch_bounds__(CB_THREADS) k_mg_coarse(const SceneDesc* __res
   // of each cell's diagonal (pressure.wgsl:77-86; 0 marks a closed cell) is tabled then too,
   // beside the previous kernel. After the wait only level lc's rhs (and p when lc = 0) is
   // read, with plain loads from L2.
-  const bool on = S.enabled;   // host-written, constant during the step
   const volatile int* act = &S.solve->active;
+  const bool on = S.enabled && !s_idle;   // enabled: host-written, constant during the step
   if (threadIdx.x == 0) {
     s_inv = 0;
     s_dir = 0;

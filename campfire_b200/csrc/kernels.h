@@ -36,7 +36,7 @@ enum TmapKind { TM_P = 0, TM_PB, TM_RHS, TM_AX, TM_AY, TM_PC, TM_PER_LEVEL };
 constexpr int TMAP_BYTES = 128;
 constexpr int COARSE_CELLS = 6144;                   // default: largest level handled by the one-CTA coarse block
 constexpr int kBlockCells = 2048;                    // the block starts no earlier than a level of this size (Engine::choose_lc)
-constexpr int kUnrolledCycles = 4;                   // fixed cycle counts up to this many are unrolled in the step graph
+constexpr int kUnrolledCycles = 12;                  // cycles laid out ahead of the step graph's loop, at most
 constexpr size_t kCoarseSmemMax = 232448 - 2048;     // dynamic shared memory of the coarse block (227 KB less static)
 constexpr int PR_TX = 32, PR_TY = 8;                 // projection
 static_assert(PR_TX == MG_TX && PR_TY == MG_TY, "the projection's tiles are counted as the level-0 multigrid tiles");

@@ -1,5 +1,5 @@
-"""Fixed cycle counts laid out in the step graph (up to four) or looped there, against kernel-by-kernel launches, and
-the coarse block's start asked for at different sizes: the same bits; the FP64 modes keep a block over level 0."""
+"""Cycles laid out in the step graph (up to twelve) and looped there, against kernel-by-kernel launches, and the
+coarse block's start asked for at different sizes: the same bits; the FP64 modes keep a block over level 0."""
 import numpy as np
 import pytest
 
@@ -26,7 +26,7 @@ def _run(nx, ny, ncycles, graphs, cells, steps=3):
 
 
 @pytest.mark.parametrize("nx,ny", [(15, 17), (32, 48), (64, 96), (112, 160)])
-@pytest.mark.parametrize("ncycles", [1, 2, 4, 5])
+@pytest.mark.parametrize("ncycles", [1, 2, 12, 13])
 def test_unrolled_cycles_equal_launched_ones(nx, ny, ncycles):
     ref, inf = _run(nx, ny, ncycles, False, 1536)
     assert inf["last_cycles"] == ncycles
@@ -35,6 +35,31 @@ def test_unrolled_cycles_equal_launched_ones(nx, ny, ncycles):
         assert i2["last_cycles"] == ncycles
         for f in FIELDS:
             assert np.array_equal(out[f], ref[f]), (graphs, cells, f)
+
+
+@pytest.mark.parametrize("mode,tol,krylov", [(cb.SOLVE_TOL, 0.3, 0), (cb.SOLVE_TOL, 1e-5, 0), (cb.SOLVE_FP64, 1e-2, 1),
+                                             (cb.SOLVE_FP64, 1e-6, 1), (cb.SOLVE_FP64, 1e-13, 1),
+                                             (cb.SOLVE_FP64, 1e-8, 3), (cb.SOLVE_FP64, 1e-9, 0)])
+def test_cycles_to_a_tolerance_equal_launched_ones(mode, tol, krylov):
+    # fewer cycles than are laid out, as many, and more (the loop's share)
+    sc = cb.generate_scene(0, 128, 192, 0.8, 44)
+    res = []
+    for graphs in (True, False):
+        g = cb.FluidSim(0, {"nx": 128, "ny": 192, "dt": sc["dt"]}, width=0.8).init()
+        load_scene(g, sc)
+        g.set_solver(mode, 1, tol, 40)
+        g.set_krylov(krylov)
+        g.set_graphs(graphs)
+        cyc = []
+        for _ in range(4):
+            g.step(1)
+            cyc.append(g.info()["last_cycles"])
+        res.append((cyc, {f: g.readBuffer(f) for f in FIELDS}, g.read_p64()))
+        g.close()
+    assert res[0][0] == res[1][0]
+    for f in FIELDS:
+        assert np.array_equal(res[0][1][f], res[1][1][f]), f
+    assert np.array_equal(res[0][2], res[1][2])
 
 
 def test_unrolled_cycles_in_a_batch():
