@@ -15,15 +15,33 @@ namespace cfg {
 
 namespace {
 
+// RN(1/x) of the divisors every cell shares, once per CTA: their quotients by div_by_rcp, the IEEE ones
+struct Rcp { float cp, sO2, dt, pr, t273; };
+
+// x / d from r = RN(1/d) also for tiny x, whose residual div_by_rcp cannot hold exactly: species
+// fade through the whole range of f32, and the advection's limiter compares them
+__device__ __forceinline__ float div_tiny(float x, float d, float r) {
+  return x != 0.f && fabsf(x) < 1e-30f ? x / d : div_by_rcp(x, d, r);
+}
+
+// what the sources read beside the diffused state; loaded before the diffusion, whose work covers
+// the round trips
+struct CellIn { float2 g; float u0, u1, v0, v1, Tadv; };
+
+// rhoDOf (gas_dev.cuh) with the shared divisors' reciprocals
+__device__ __forceinline__ float rhoD(const cfg_params& P, const Rcp& R, float T) {
+  const float v = 1.716e-5f * powf(div_by_rcp(T, 273.15f, R.t273), 1.5f) * (float)(273.15 + 110.4) / (T + 110.4f);
+  return div_by_rcp(v, P.Pr, R.pr) * P.diffMult;
+}
+
 // sources.wgsl:34-157 for one gas cell; returns false for a cell inside wood
 struct SrcOut { float T; float4 Y; float S, qrel, qrad, tpeak; bool solid; };
 
 // Tamb4 = powf(P.Tamb, 4) (the radiation's ambient term, the same for every cell of the scene)
-__device__ __forceinline__ SrcOut sources_cell(const SceneDesc& S, const cfg_params& P, int i, int j, float Tc, float4 Yc,
-                                               float Tadv, float Tamb4) {
+__device__ __forceinline__ SrcOut sources_cell(const SceneDesc& S, const cfg_params& P, const Rcp& R, const CellIn& in, int i, int j,
+                                               float Tc, float4 Yc, float Tamb4) {
   SrcOut o; o.qrel = 0.f; o.qrad = 0.f; o.tpeak = 0.f; o.solid = false; o.S = 0.f;
-  const int k = j * S.pc + i;
-  const float2 g = __ldg(S.cellG + k);
+  const float2 g = in.g;
   const float sdf = g.x;
   const uint32_t sid = __float_as_uint(g.y);
   float massSrc = 0.f;
@@ -45,7 +63,7 @@ __device__ __forceinline__ SrcOut sources_cell(const SceneDesc& S, const cfg_par
     const float band = (float)__ldg(S.faceW + sid) / 1.0e8f;
     const float w = fmaxf(0.f, 1.f - fabsf(sdf - dx) / dx) / dx * (2.f * half) / fmaxf(band, 1e-6f);
     const float rho = rhoOf(P, Tc);
-    const float kg = rhoDOf(P, 0.5f * (Tc + Ts)) * P.cp;
+    const float kg = rhoD(P, R, 0.5f * (Tc + Ts)) * P.cp;
     const float dist = fmaxf(sdf, 0.5f * dx);
     const float rate = kg * w / (dist * rho * P.cp);
     const float dTc = (Ts - Tc) * (1.f - expf(-rate * dt));
@@ -93,19 +111,27 @@ __device__ __forceinline__ SrcOut sources_cell(const SceneDesc& S, const cfg_par
   #pragma unroll 1
   for (int s = 0; s < 8; s++) {
     const float wr = P.reactB * rho0 * Yc.x * Yc.y * expf(-P.reactTa / Tc);
-    const float dF = fminf(wr * h, fminf(Yc.x, Yc.y / P.sO2));
-    Yc = make_float4(Yc.x + -dF, Yc.y + -P.sO2 * dF, Yc.z + (1.f + P.sO2) * dF, Yc.w + 0.f);
-    Tc += dF * P.dHc / P.cp;
+    const float dF = fminf(wr * h, fminf(Yc.x, div_tiny(Yc.y, P.sO2, R.sO2)));
+    const float4 Yn = make_float4(Yc.x + -dF, Yc.y + -P.sO2 * dF, Yc.z + (1.f + P.sO2) * dF, Yc.w + 0.f);
+    const float Tn = Tc + div_tiny(dF * P.dHc, P.cp, R.cp);
     burned += dF;
+    // cold or fuel-free gas: a sub-step that leaves the state as it was repeats itself
+    const bool still = Yn.x == Yc.x && Yn.y == Yc.y && Yn.z == Yc.z && Tn == Tc;
+    Yc = Yn; Tc = Tn;
+    if (still) {
+      for (s++; s < 8; s++) burned += dF;
+      break;
+    }
   }
   // :122-128 soot formation and oxidation
   const float dSf = fminf(P.sootFormA * expf(-P.sootFormTa / Tc) * Yc.x * dt, Yc.x);
   Yc = make_float4(Yc.x + -dSf, Yc.y + 0.f, Yc.z + 0.f, Yc.w + dSf);
-  const float dSo = fminf(P.sootOxA * Yc.w * Yc.y * expf(-P.sootOxTa / Tc) * dt, fminf(Yc.w, Yc.y / P.sO2));
+  const float dSo = fminf(P.sootOxA * Yc.w * Yc.y * expf(-P.sootOxTa / Tc) * dt,
+                          fminf(Yc.w, div_tiny(Yc.y, P.sO2, R.sO2)));
   Yc = make_float4(Yc.x + 0.f, Yc.y + -P.sO2 * dSo, Yc.z + (1.f + P.sO2) * dSo, Yc.w + -dSo);
-  Tc += dSo * P.dHc / P.cp;
+  Tc += div_tiny(dSo * P.dHc, P.cp, R.cp);
   burned += dSo;
-  o.qrel = rho0 * burned * P.dHc / dt;
+  o.qrel = div_tiny(rho0 * burned * P.dHc, dt, R.dt);
   // :130-136 optically thin radiation, linearised implicit
   const float r1 = rhoOf(P, Tc);
   const float fv = r1 * Yc.w / P.sootDensity;
@@ -115,38 +141,54 @@ __device__ __forceinline__ SrcOut sources_cell(const SceneDesc& S, const cfg_par
   const float dTr = o.qrad * dt / (r1 * P.cp) / (1.f + 16.f * kap * P.sigma * T3 * dt / (r1 * P.cp));
   Tc -= dTr;
   // :140-148 entrainment of ambient air through the front/back faces
-  const float ucx = 0.5f * (__ldg(S.U + j * S.pu + i) + __ldg(S.U + j * S.pu + i + 1));
-  const float ucy = 0.5f * (__ldg(S.V + j * S.pc + i) + __ldg(S.V + (j + 1) * S.pc + i));
+  const float ucx = 0.5f * (in.u0 + in.u1), ucy = 0.5f * (in.v0 + in.v1);
   const float me = 2.f * P.exchAlpha * sqrtf(ucx * ucx + ucy * ucy) * P.rhoAmb / P.depth;
   if (me > 0.f) {
     const float madd = me * dt;
     const float r = rhoOf(P, Tc);
     const float4 a = ambY(P);
-    Yc = make_float4((r * Yc.x + madd * a.x) / (r + madd), (r * Yc.y + madd * a.y) / (r + madd),
-                     (r * Yc.z + madd * a.z) / (r + madd), (r * Yc.w + madd * a.w) / (r + madd));
-    Tc = (r * Tc + madd * P.Tamb) / (r + madd);
+    const float m = r + madd, rm = __frcp_rn(m);   // five quotients by one divisor
+    Yc = make_float4(div_tiny(r * Yc.x + madd * a.x, m, rm), div_tiny(r * Yc.y + madd * a.y, m, rm),
+                     div_tiny(r * Yc.z + madd * a.z, m, rm), div_tiny(r * Yc.w + madd * a.w, m, rm));
+    Tc = div_by_rcp(r * Tc + madd * P.Tamb, m, rm);
     massSrc += me;
   }
   // :150-156
   Tc = fmaxf(Tc, 0.5f * P.Tamb);
   Yc = max4(Yc, make_float4(0.f, 0.f, 0.f, 0.f));
-  o.S = massSrc / rhoOf(P, Tc) + logf(Tc / Tadv) / dt;
+  o.S = massSrc / rhoOf(P, Tc) + div_by_rcp(logf(Tc / in.Tadv), dt, R.dt);
   o.T = Tc; o.Y = Yc; o.tpeak = Tc;
   return o;
 }
 
 }  // namespace
 
-// NMAX: largest diffusion sub-step count this instantiation handles (halo NMAX)
+// threads: one per cell of the tile and its one-cell ring, so that with one sub-step (the ordinary
+// case) the load, the faces and the cells are one round each
+template <int TX, int TY>
+constexpr int ds_threads() { return ((TX + 2) * (TY + 2) + 31) / 32 * 32; }
+
+// NMAX: largest diffusion sub-step count this instantiation handles (halo NMAX).
+// Each sub-step first evaluates every face's f rho D once (diffuse.wgsl has each cell evaluate its
+// four faces, so every face twice; the two results are equal), then updates the cells from the
+// faces. Bound by the arithmetic of powf and of the sources' chain of eight dependent sub-steps.
+// A step with one sub-step: 160x224 90.7 -> 88.7 us, 224x320 95.7 -> 94.5, 32x48 71.8 -> 70.7, the
+// 64-scene batch 4706 -> 4699; with three: 352x512 144.0 -> 142.9. Four CTAs of 352 threads per
+// SM with one sub-step (40 registers, 28 bytes of spill): three cost the batch 0.5%, five the
+// small grids 1-3%.
 template <int TX, int TY, int NMAX, bool SOURCES, bool DIFFUSION>
-__global__ void __launch_bounds__(256) k_diffuse_sources(const SceneDesc* __restrict__ scenes, const Work* __restrict__ work) {
+__global__ void __launch_bounds__(ds_threads<TX, TY>(), TX * TY == 256 ? (NMAX == 1 ? 4 : 3) : 2) k_diffuse_sources(const SceneDesc* __restrict__ scenes, const Work* __restrict__ work) {
   constexpr int RW = TX + 2 * NMAX, RH = TY + 2 * NMAX;
-  // the ping-pong state of tile + halo in dynamic shared memory (ds_smem_bytes: above 48 KB for
-  // the larger tiles at 5 sub-steps)
+  // the ping-pong state of tile + halo and the faces' coefficients in dynamic shared memory
+  // (ds_smem_bytes: above 48 KB for the larger tiles at 5 sub-steps)
   extern __shared__ __align__(16) unsigned char ds_smem[];
   float4 (*sY)[RH * RW] = reinterpret_cast<float4 (*)[RH * RW]>(ds_smem);
   float (*sT)[RH * RW] = reinterpret_cast<float (*)[RH * RW]>(ds_smem + 2 * RH * RW * sizeof(float4));
+  float* sAx = sT[0] + 2 * RH * RW;   // west face of region cell r
+  float* sAy = sAx + RH * RW;         // south face
   __shared__ float rq[TY * TX], rr[TY * TX], rt[TY * TX];
+  __shared__ Rcp s_rcp;
+  __shared__ int s_acc[3];
 
   const Work w = work[blockIdx.x];
   const SceneDesc& S = scenes[w.scene];
@@ -167,7 +209,21 @@ __global__ void __launch_bounds__(256) k_diffuse_sources(const SceneDesc* __rest
     sT[0][e] = __ldg(Tin + j * pc + i);
     sY[0][e] = __ldg(Yin + j * pc + i);
   }
+  CellIn in{};
+  const int oi = x0 + (int)threadIdx.x % TX, oj = y0 + (int)threadIdx.x / TX;
+  const bool own = threadIdx.x < TX * TY && oi < nx && oj < ny;
+  if (SOURCES && own) {
+    const int k = oj * pc + oi;
+    in.g = __ldg(S.cellG + k);
+    in.u0 = __ldg(S.U + oj * pu + oi); in.u1 = __ldg(S.U + oj * pu + oi + 1);
+    in.v0 = __ldg(S.V + k); in.v1 = __ldg(S.V + k + pc);
+    in.Tadv = __ldg(S.T2 + k);
+  }
+  if (threadIdx.x < 3) s_acc[threadIdx.x] = 0;
+  if (threadIdx.x == blockDim.x - 1)
+    s_rcp = Rcp{__frcp_rn(P.cp), __frcp_rn(P.sO2), __frcp_rn(P.dt), __frcp_rn(P.Pr), __frcp_rn(273.15f)};
   __syncthreads();
+  const Rcp R = s_rcp;
 
   // ---- diffusion sub-steps (diffuse.wgsl:18-50), buffer ping-pong in shared memory
   const float c0 = S.diff_dt;
@@ -175,28 +231,41 @@ __global__ void __launch_bounds__(256) k_diffuse_sources(const SceneDesc* __rest
   for (int s = 1; s <= n; s++) {
     const int xa = max(x0 - n + s, 0), xb = min(x0 + TX + n - s, nx);
     const int ya = max(y0 - n + s, 0), yb = min(y0 + TY + n - s, ny);
-    const int W = xb - xa, Hh = yb - ya;
     const float* Ti = sT[cur]; const float4* Yi = sY[cur];
     float* To = sT[cur ^ 1]; float4* Yo = sY[cur ^ 1];
-    for (int e = threadIdx.x; e < W * Hh; e += blockDim.x) {
-      const int i = xa + e % W, j = ya + e / W;
-      const int r = (j - ry0) * RW + (i - rx0);
+    // the faces west of columns xa..xb and south of rows ya..yb; none at the domain's edges
+    for (int r = threadIdx.x; r < RH * RW; r += blockDim.x) {
+      const int i = rx0 + r % RW, j = ry0 + r / RW;
+      if (i < xa || i > xb || j < ya || j > yb) continue;
+      if (j < yb) {
+        const float f = i > 0 && i < nx ? __ldg(S.fx + j * pu + i) : 0.f;
+        sAx[r] = f > 0.f ? f * rhoD(P, R, 0.5f * (Ti[r] + Ti[r - 1])) : 0.f;
+      }
+      if (i < xb) {
+        const float f = j > 0 && j < ny ? __ldg(S.fy + j * pc + i) : 0.f;
+        sAy[r] = f > 0.f ? f * rhoD(P, R, 0.5f * (Ti[r] + Ti[r - RW])) : 0.f;
+      }
+    }
+    __syncthreads();
+    for (int r = threadIdx.x; r < RH * RW; r += blockDim.x) {
+      const int i = rx0 + r % RW, j = ry0 + r / RW;
+      if (i < xa || i >= xb || j < ya || j >= yb) continue;
       const float T0 = Ti[r]; const float4 Y0 = Yi[r];
       float sTa = 0.f; float sYx = 0.f, sYy = 0.f, sYz = 0.f;
-      #define CFG_DIFF_FACE(fval, roff)                                          \
+      // west, east, south, north; a closed face's coefficient is zero
+      #define CFG_DIFF_FACE(coef, roff)                                         \
         {                                                                       \
-          const float f = (fval);                                               \
-          if (f > 0.f) {                                                        \
+          const float a = (coef);                                               \
+          if (a > 0.f) {                                                        \
             const float Tn = Ti[r + (roff)]; const float4 Yn = Yi[r + (roff)];  \
-            const float a = f * rhoDOf(P, 0.5f * (T0 + Tn));                    \
             sTa += a * (Tn - T0);                                               \
             sYx += a * (Yn.x - Y0.x); sYy += a * (Yn.y - Y0.y); sYz += a * (Yn.z - Y0.z); \
           }                                                                     \
         }
-      if (i > 0) CFG_DIFF_FACE(__ldg(S.fx + j * pu + i), -1)
-      if (i < nx - 1) CFG_DIFF_FACE(__ldg(S.fx + j * pu + i + 1), 1)
-      if (j > 0) CFG_DIFF_FACE(__ldg(S.fy + j * pc + i), -RW)
-      if (j < ny - 1) CFG_DIFF_FACE(__ldg(S.fy + (j + 1) * pc + i), RW)
+      CFG_DIFF_FACE(sAx[r], -1)
+      CFG_DIFF_FACE(sAx[r + 1], 1)
+      CFG_DIFF_FACE(sAy[r], -RW)
+      CFG_DIFF_FACE(sAy[r + RW], RW)
       #undef CFG_DIFF_FACE
       const float c = c0 / (rhoOf(P, T0) * P.dx * P.dx);
       To[r] = T0 + c * sTa;
@@ -207,16 +276,14 @@ __global__ void __launch_bounds__(256) k_diffuse_sources(const SceneDesc* __rest
   }
 
   // ---- sources on the tile cells (or write the diffused state)
-  const float Tamb4 = powf(P.Tamb, 4.f);
-  for (int e = threadIdx.x; e < TX * TY; e += blockDim.x) {
-    const int i = x0 + e % TX, j = y0 + e / TX;
+  if (threadIdx.x < TX * TY) {
+    const int e = threadIdx.x;
     float q = 0.f, qr = 0.f, tp = 0.f;
-    if (i < nx && j < ny) {
-      const int r = (j - ry0) * RW + (i - rx0);
-      const int k = j * pc + i;
+    if (own) {
+      const int r = (oj - ry0) * RW + (oi - rx0), k = oj * pc + oi;
       const float Tc = sT[cur][r]; const float4 Yc = sY[cur][r];
       if (SOURCES) {
-        const SrcOut o = sources_cell(S, P, i, j, Tc, Yc, __ldg(S.T2 + k), Tamb4);
+        const SrcOut o = sources_cell(S, P, R, in, oi, oj, Tc, Yc, powf(P.Tamb, 4.f));
         S.T[k] = o.T; S.Y[k] = o.Y;
         S.SQ[k] = o.solid ? make_float2(0.f, 0.f) : make_float2(o.S, o.qrel);
         q = o.qrel; qr = o.qrad; tp = o.tpeak;
@@ -242,21 +309,25 @@ __global__ void __launch_bounds__(256) k_diffuse_sources(const SceneDesc* __rest
       vr = vr + __shfl_down_sync(0xffffffffu, vr, o);
       vt = fmaxf(vt, __shfl_down_sync(0xffffffffu, vt, o));
     }
-    // a block entirely outside the domain still adds round(0) = 0, as the WGSL does
+    // each 8x8 block rounds to fixed point as the WGSL's workgroups do; the integers of the CTA's
+    // blocks are added here first (every CTA of a scene goes to the same three words)
     if (lane == 0) {
-      atomicAdd(S.acc + ACC_GLOBAL, wgsl_i32_round(vq * 1.0e3f));
-      atomicAdd(S.acc + ACC_GLOBAL + 1, wgsl_i32_round(vr * 1.0e3f));
-      atomicMax(S.acc + ACC_GLOBAL + 2, wgsl_i32(vt));
+      atomicAdd(s_acc, wgsl_i32_round(vq * 1.0e3f));
+      atomicAdd(s_acc + 1, wgsl_i32_round(vr * 1.0e3f));
+      atomicMax(s_acc + 2, wgsl_i32(vt));
     }
   }
+  __syncthreads();
+  if (threadIdx.x < 2 && s_acc[threadIdx.x] != 0) atomicAdd(S.acc + ACC_GLOBAL + threadIdx.x, s_acc[threadIdx.x]);
+  if (threadIdx.x == 2) atomicMax(S.acc + ACC_GLOBAL + 2, s_acc[2]);
 }
 
 template <int TX, int TY, int NMAX>
-constexpr size_t ds_smem_bytes() { return (size_t)2 * (TX + 2 * NMAX) * (TY + 2 * NMAX) * (sizeof(float4) + sizeof(float)); }
+constexpr size_t ds_smem_bytes() { return (size_t)(TX + 2 * NMAX) * (TY + 2 * NMAX) * (2 * sizeof(float4) + 4 * sizeof(float)); }
 
 template <int TX, int TY, int NMAX, bool SRC, bool DIF>
 static void ds_launch(const SceneDesc* scenes, const Work* work, int ntiles, cudaStream_t st) {
-  k_diffuse_sources<TX, TY, NMAX, SRC, DIF><<<ntiles, 256, ds_smem_bytes<TX, TY, NMAX>(), st>>>(scenes, work);
+  k_diffuse_sources<TX, TY, NMAX, SRC, DIF><<<ntiles, ds_threads<TX, TY>(), ds_smem_bytes<TX, TY, NMAX>(), st>>>(scenes, work);
 }
 template <int TX, int TY>
 static void ds_launch_shape(const SceneDesc* scenes, const Work* work, int ntiles, int max_sub, bool with_sources,
