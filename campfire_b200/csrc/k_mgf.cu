@@ -150,142 +150,232 @@ __device__ __forceinline__ bool tile_wait2(uint64_t* bar, SolveCtl* ctl, F&& bet
 }
 
 
-// The four colour passes of a fused kernel with every cell's stencil in registers. Pass k
-// (1..4) covers [x0-H+k, x0+TX+H-k) x [y0-H+k, y0+TY+H-k) clipped to the level, with colour
-// (first + k - 1) & 1; thread t owns slots t and t + 256 of each colour in pass 1's region
-// (the largest; 20 cells of a colour per row). tile_stencils builds their stencils from the
-// coefficients alone (the four coefficients, zero for a neighbour outside the level, the
-// diagonal, its correctly rounded reciprocal, the passes that include the cell, whether it
-// is a tile cell); tile_passes adds rhs h2 once the state has landed and updates the cells
-// by pressure.wgsl:87-94, dividing by div_by_rcp.
-struct TCell { float w, e, s, n, rh, diag, rcp; int kp, fl; };   // fl: 1 a tile cell; 16 << k: pass k
-constexpr int SM_W1 = MGF_TX + 2 * MGF_H - 2, SM_H1 = MGF_TY + 2 * MGF_H - 2;   // pass 1's region
-__device__ __forceinline__ void tile_stencils(const Tile& t, const LevelDesc& L, int x0, int y0, int first,
-                                              TCell (&c)[2][2]) {
-  constexpr int HALF = SM_W1 / 2;
-  static_assert(SM_W1 % 2 == 0 && HALF * SM_H1 <= 2 * 256, "two slots of a colour per thread");
-  const int ib = x0 - MGF_H + 1, jb = y0 - MGF_H + 1;
-  #pragma unroll
-  for (int col = 0; col < 2; col++)
-    #pragma unroll
-    for (int m = 0; m < 2; m++) {
-      TCell& q = c[col][m];
-      q.fl = 0;
-      const int sl = threadIdx.x + 256 * m;
-      if (sl >= HALF * SM_H1) continue;
-      const int r = sl / HALF, j = jb + r, i = ib + ((ib + j + col) & 1) + 2 * (sl - r * HALF);
-      if (i < 0 || i >= L.nx || j < 0 || j >= L.ny) continue;
-      // pass k (1..4) covers the cells at distance >= k from the edge of the region
-      // [x0-H, x0+TX+H) x [y0-H, y0+TY+H), and has colour (first + k - 1) & 1: passes 1, 3
-      // or 2, 4 for this cell's colour, up to its distance; distance >= H: a tile cell
-      const int d = min(min(i - (x0 - MGF_H), x0 + MGF_TX + MGF_H - 1 - i),
-                        min(j - (y0 - MGF_H), y0 + MGF_TY + MGF_H - 1 - j));
-      const int pm = (((first ^ col) & 1) ? (64 | 256) : (32 | 128)) & (((2 << min(d, 4)) - 2) << 4);
-      if (!pm) continue;
-      const int k = t.c(i, j);
-      q.kp = k;
-      const float w = t.ax[k], e = t.ax[k + 1], s = t.ay[k], n = t.ay[k + MGF_BW];
-      float diag = 0.f;
-      if (i > 0) diag += w; else diag += 2.f * w;
-      if (i < L.nx - 1) diag += e; else diag += 2.f * e;
-      if (j > 0) diag += s;
-      if (j < L.ny - 1) diag += n; else diag += 2.f * n;
-      q.diag = diag;
-      q.rcp = diag > 0.f ? __frcp_rn(diag) : 0.f;
-      // a neighbour outside the level contributes nothing (pressure.wgsl:77-85): its
-      // coefficient is zero in the passes' sums, whose values outside the level are zero
-      q.w = i > 0 ? w : 0.f;
-      q.e = i < L.nx - 1 ? e : 0.f;
-      q.s = j > 0 ? s : 0.f;
-      q.n = j < L.ny - 1 ? n : 0.f;
-      q.fl = pm | (d >= MGF_H ? 1 : 0);
-    }
+// ---- packed pairs of f32: one instruction for two operations, each rounded as its scalar form.
+// A product is the fused multiply-add with -0 (a b + -0 rounds to a b, signs of zero kept), its -0
+// an argument of the kernel: the assembler contracts mul.rn.f32x2 with an add.rn.f32x2 that
+// follows it, whatever -fmad says, and a fused one with a -0 that it can see as well.
+typedef unsigned long long f2;
+__device__ __forceinline__ f2 pk(float a, float b) { f2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
+__device__ __forceinline__ void upk(f2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ f2 add2(f2 a, f2 b) { f2 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) { f2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
+__device__ __forceinline__ f2 mul2(f2 a, f2 b, f2 nz) { return fma2(a, b, nz); }
+__device__ __forceinline__ f2 lds2(const float* p) { const float2 v = *reinterpret_cast<const float2*>(p); return pk(v.x, v.y); }
+__device__ __forceinline__ void sts2(float* p, f2 v) { float2 w; upk(v, w.x, w.y); *reinterpret_cast<float2*>(p) = w; }
+
+// The four colour passes of a fused kernel. Thread t owns item t of pass 1's region (40 x 24 cells,
+// 240 items): the four cells (base..base+3, j) of one row, base even, which are two cells of each
+// colour. Their stencils stay in registers as packed pairs by colour, and so do the cells' own
+// values. The tile's p is held twice 26 columns to a row, red cells and black ones apart (column
+// pair c of box row r: sp[r SPW + c] and sp[r SPW + SPB + c]): a pass then reads the other colour
+// of the rows below and above as one aligned pair each and one neighbour beside the item; the
+// rest of the row is the item's own. Passes 2-4 update the whole region again: a cell at distance d from its
+// edge is exact through pass d, a later update there only spoils values that no cell
+// needed later reads (pass k of a cell at distance >= k reads cells at distance >= k - 1). Cells
+// outside the level and closed ones have zeros throughout and stay zero. The sums leave out
+// the leading +0 of pressure.wgsl:77-85, which changes no value. The quotient is div_by_rcp's.
+constexpr int RG_W = MGF_TX + 2 * MGF_H - 2, RG_H = MGF_TY + 2 * MGF_H - 2;   // pass 1's region
+constexpr int RG_IW = RG_W / 4, RG_N = RG_IW * RG_H;                          // items per row, items
+static_assert(RG_W % 4 == 0 && RG_N <= 256 && MGF_H == 5 && MGF_SX == 8, "one item per thread");
+constexpr int SPB = 26, SPW = 2 * SPB, SP_N = MGF_BH * SPW;   // 52 words per row: pairs of 3 rows hit 32 banks evenly
+struct Item {
+  int r, j, base, k, c;   // region row, level row, first cell's level column, box index, column pair
+  bool on, odd;           // owns an item; j odd: the red cells are base+1, base+3
+};
+__device__ __forceinline__ Item item_of(int x0, int y0) {
+  Item q;
+  q.on = threadIdx.x < RG_N;
+  q.r = threadIdx.x / RG_IW;
+  const int a = threadIdx.x - q.r * RG_IW;
+  q.j = y0 - MGF_H + 1 + q.r;
+  q.base = x0 - MGF_H + 1 + 4 * a;
+  q.k = (q.r + 1) * MGF_BW + MGF_SX - MGF_H + 1 + 4 * a;
+  q.c = (MGF_SX - MGF_H + 1) / 2 + 2 * a;
+  q.odd = q.j & 1;
+  return q;
 }
-// off of pressure.wgsl:77-85 from the slot's stencil: every neighbour's term is added in the
-// reference's order (west, east, south, north); a missing neighbour's term is an exact zero,
-// and adding it to a sum that started at +0 leaves the sum's bits unchanged
-__device__ __forceinline__ float tcell_off(const Tile& t, const TCell& q) {
-  float off = 0.f;
-  off += q.w * t.p[q.kp - 1];
-  off += q.e * t.p[q.kp + 1];
-  off += q.s * t.p[q.kp - MGF_BW];
-  off += q.n * t.p[q.kp + MGF_BW];
+// whether the item lies in the tile
+__device__ __forceinline__ bool in_tile(const Item& q, int x0, int y0) {
+  return q.on && q.base >= x0 && q.base < x0 + MGF_TX && q.j >= y0 && q.j < y0 + MGF_TY;
+}
+// four values in column order as pairs by colour, and back
+__device__ __forceinline__ void by_colour(const Item& q, const float (&v)[4], f2 (&c)[2]) {
+  const f2 e = pk(v[0], v[2]), o = pk(v[1], v[3]);
+  c[0] = q.odd ? o : e; c[1] = q.odd ? e : o;
+}
+__device__ __forceinline__ float4 in_order(const Item& q, const f2 (&c)[2]) {
+  float4 v;
+  upk(q.odd ? c[1] : c[0], v.x, v.z);
+  upk(q.odd ? c[0] : c[1], v.y, v.w);
+  return v;
+}
+struct Sten { f2 w[2], e[2], s[2], n[2], nd[2], rc[2], nrh[2], nz; };   // nd: -diag, rc: RN(1/diag), nrh: -(rhs h2), nz: -0
+// the stencils from the coefficients alone
+__device__ __forceinline__ void item_stencils(const Tile& t, const LevelDesc& L, const Item& q, Sten& c) {
+  float w[4], e[4], s[4], n[4], nd[4], rc[4];
+  #pragma unroll
+  for (int m = 0; m < 4; m++) w[m] = e[m] = s[m] = n[m] = nd[m] = rc[m] = 0.f;
+  if (q.on && (unsigned)q.j < (unsigned)L.ny) {
+    const float4 A = *reinterpret_cast<const float4*>(t.ax + q.k), Sv = *reinterpret_cast<const float4*>(t.ay + q.k),
+                 Nv = *reinterpret_cast<const float4*>(t.ay + q.k + MGF_BW);
+    const float a[5] = {A.x, A.y, A.z, A.w, t.ax[q.k + 4]}, sv[4] = {Sv.x, Sv.y, Sv.z, Sv.w}, nv[4] = {Nv.x, Nv.y, Nv.z, Nv.w};
+    #pragma unroll
+    for (int m = 0; m < 4; m++) {
+      const int i = q.base + m;
+      float d = i > 0 ? a[m] : 2.f * a[m];
+      d += i < L.nx - 1 ? a[m + 1] : 2.f * a[m + 1];
+      if (q.j > 0) d += sv[m];
+      d += q.j < L.ny - 1 ? nv[m] : 2.f * nv[m];
+      if ((unsigned)i < (unsigned)L.nx && d > 0.f) {
+        w[m] = a[m]; e[m] = a[m + 1]; s[m] = sv[m]; n[m] = nv[m]; nd[m] = -d; rc[m] = __frcp_rn(d);
+      }
+    }
+  }
+  by_colour(q, w, c.w); by_colour(q, e, c.e); by_colour(q, s, c.s); by_colour(q, n, c.n);
+  by_colour(q, nd, c.nd); by_colour(q, rc, c.rc);
+}
+// the item's rhs (column order) into the stencils; kept apart for the residual where `rhs` asks
+__device__ __forceinline__ void item_rhs(const Item& q, float h2, const float4 r, Sten& c, f2* rhs = nullptr) {
+  const float v[4] = {r.x, r.y, r.z, r.w};
+  f2 x[2];
+  by_colour(q, v, x);
+  const f2 m = pk(-h2, -h2);
+  c.nrh[0] = mul2(x[0], m, c.nz); c.nrh[1] = mul2(x[1], m, c.nz);
+  if (rhs) { rhs[0] = x[0]; rhs[1] = x[1]; }
+}
+// the sum of coefficient times neighbour for the item's cells of colour col, in the reference's
+// order (west, east, south, north); own: the item's cells of the other colour
+__device__ __forceinline__ f2 item_off(const float* sp, const Item& q, const Sten& c, int col, f2 own) {
+  const float* o = sp + (q.r + 1) * SPW + (1 - col) * SPB + q.c;   // the other colour's row
+  const bool hi = q.odd != (col == 1);   // this colour's cells are base+1, base+3
+  float o0, o1;
+  upk(own, o0, o1);
+  const float x = o[hi ? 2 : -1], y = hi ? o1 : o0;
+  f2 off = mul2(c.w[col], pk(hi ? o0 : x, y), c.nz);
+  off = add2(off, mul2(c.e[col], pk(y, hi ? x : o1), c.nz));
+  off = add2(off, mul2(c.s[col], lds2(o - SPW), c.nz));
+  off = add2(off, mul2(c.n[col], lds2(o + SPW), c.nz));
   return off;
 }
-__device__ __forceinline__ void tile_passes(const Tile& t, const LevelDesc& L, int first, TCell (&c)[2][2]) {
+__device__ __forceinline__ f2 quot2(f2 x, f2 nd, f2 r, f2 nz) {   // div_by_rcp; nd: minus the divisor
+  const f2 q0 = mul2(x, r, nz);
+  return fma2(fma2(q0, nd, x), r, q0);
+}
+// p[col]: the item's own values, also in sp; on return the smoothed ones
+__device__ __forceinline__ void item_passes(float* sp, const Item& q, const Sten& c, int first, f2 (&p)[2]) {
   #pragma unroll
-  for (int col = 0; col < 2; col++)
-    #pragma unroll
-    for (int m = 0; m < 2; m++)
-      if (c[col][m].fl) c[col][m].rh = t.rhs[c[col][m].kp] * L.h2;
-  #pragma unroll
-  for (int k = 1; k <= 4; k++) {
-    const int col = (first + k - 1) & 1;
-    float v[2];
-    #pragma unroll
-    for (int m = 0; m < 2; m++) {
-      const TCell& q = c[col][m];
-      if (!(q.fl & (16 << k))) continue;
-      const float off = tcell_off(t, q);
-      v[m] = q.diag > 0.f ? mgc::div_by_rcp(off - q.rh, q.diag, q.rcp) : 0.f;
+  for (int k = 0; k < 4; k++) {
+    const int col = (first + k) & 1;
+    if (q.on) {
+      p[col] = quot2(add2(item_off(sp, q, c, col, p[1 - col]), c.nrh[col]), c.nd[col], c.rc[col], c.nz);
+      sts2(sp + (q.r + 1) * SPW + col * SPB + q.c, p[col]);
     }
-    #pragma unroll
-    for (int m = 0; m < 2; m++)
-      if (c[col][m].fl & (16 << k)) t.p[c[col][m].kp] = v[m];
     __syncthreads();
   }
 }
+__device__ __forceinline__ void put_item(float* sp, const Item& q, const f2 (&p)[2]) {
+  sts2(sp + (q.r + 1) * SPW + q.c, p[0]);
+  sts2(sp + (q.r + 1) * SPW + SPB + q.c, p[1]);
+}
+// The ring of one cell about pass 1's region, whose values pass 1 reads: ring cell e's box row and
+// column (two rows of 42, then two columns of 24)
+constexpr int RING_N = 2 * (RG_W + 2) + 2 * RG_H;
+static_assert(RING_N <= 256, "one ring cell per thread");
+__device__ __forceinline__ void ring_cell(int e, int& br, int& bc) {
+  constexpr int w = RG_W + 2;
+  if (e < 2 * w) { br = e < w ? 0 : RG_H + 1; bc = MGF_SX - MGF_H + (e < w ? e : e - w); }
+  else { e -= 2 * w; br = 1 + (e >> 1); bc = MGF_SX - MGF_H + ((e & 1) ? RG_W + 1 : 0); }
+}
+// where box cell (br, bc) of the tile at (sx, sy) lies in sp
+__device__ __forceinline__ int sp_at(int br, int bc, int sx, int sy) {
+  return br * SPW + (((sx + bc + sy + br) & 1) ? SPB : 0) + (bc >> 1);
+}
+// p of the box into sp as it is (level 0 from a start that is not zero), or zeros
+__device__ __forceinline__ void stage_sp(const Tile& t, float* sp, const Item& q, f2 (&p)[2]) {
+  if (q.on) {
+    const float4 v = *reinterpret_cast<const float4*>(t.p + q.k);
+    const float a[4] = {v.x, v.y, v.z, v.w};
+    by_colour(q, a, p);
+    put_item(sp, q, p);
+  }
+  if (threadIdx.x < RING_N) {
+    int br, bc;
+    ring_cell(threadIdx.x, br, bc);
+    sp[sp_at(br, bc, t.sx, t.sy)] = t.p[br * MGF_BW + bc];
+  }
+}
+__device__ __forceinline__ void zero_sp(float* sp, f2 (&p)[2]) {
+  for (int e = threadIdx.x; e < SP_N / 4; e += 256) reinterpret_cast<float4*>(sp)[e] = make_float4(0.f, 0.f, 0.f, 0.f);
+  p[0] = p[1] = 0ull;
+}
+static_assert(SP_N % 4 == 0, "filled by float4");
 
-// The up kernel's prolongation (pressure.wgsl:116-129) over the region [x0-H, x0+TX+H) x
-// [y0-H, y0+TY+H); with one scene split in two. prolong_plan (from the coefficients and the level
-// sizes alone, beside the stencils before the wait) packs for element e = threadIdx.x + 256 m: the fine cell's box index
-// (bits 0-10), the index in the coarse box of its own coarse cell (11-19), the steps to the other
-// coarse column and row of its bilinear stencil plus one (20-21, 22-23), whether the cell is open
-// (24) and whether it lies in the level (25). prolong_apply adds the interpolated correction once
-// the coarse box has landed: a closed cell adds +0, as pressure.wgsl:129 has it.
-constexpr int PR_W = MGF_TX + 2 * MGF_H, PR_H = MGF_TY + 2 * MGF_H, PR_N = (PR_W * PR_H + 255) / 256;
+// The up kernel's prolongation (pressure.wgsl:116-129) over the region and its ring: the bilinear
+// correction from the coarse box at (cx, cy), added to open cells. An item's four cells lie over two
+// coarse cells; its sums are formed as packed pairs (cells 0, 1 and 2, 3).
+__device__ __forceinline__ void prolong_item(const Tile& t, const LevelDesc& C, const Item& q, const Sten& c, int cx, int cy,
+                                             const float* scp, f2 (&p)[2]) {
+  const int I = q.base / 2, J = q.j / 2;
+  const int J2 = min(max(J + ((q.j & 1) ? 1 : -1), 0), C.ny - 1);
+  const int il = max(I - 1, 0), ir = min(I + 2, C.nx - 1), im = min(I + 1, C.nx - 1);
+  const float* a = scp + (J - cy) * MGF_CBW - cx;
+  const float* b = scp + (J2 - cy) * MGF_CBW - cx;
+  const float a0 = a[I], a1 = a[im], al = a[il], ar = a[ir], b0 = b[I], b1 = b[im], bl = b[il], br = b[ir];
+  const f2 k0 = pk(0.5625f, 0.5625f), k1 = pk(0.1875f, 0.1875f), k2 = pk(0.0625f, 0.0625f);
+  const f2 z = c.nz;
+  f2 u = add2(add2(mul2(k0, pk(a0, a0), z), mul2(k1, add2(pk(al, a1), pk(b0, b0)), z)), mul2(k2, pk(bl, b1), z));
+  f2 v = add2(add2(mul2(k0, pk(a1, a1), z), mul2(k1, add2(pk(a0, ar), pk(b1, b1)), z)), mul2(k2, pk(b0, br), z));
+  float x[4];
+  upk(u, x[0], x[1]);
+  upk(v, x[2], x[3]);
+  f2 d[2];
+  by_colour(q, x, d);
+  // closed cells and cells outside the level (zero diagonal) add nothing
+  #pragma unroll
+  for (int col = 0; col < 2; col++) {
+    float r0, r1, x0, x1;
+    upk(c.rc[col], r0, r1);
+    upk(d[col], x0, x1);
+    d[col] = pk(r0 != 0.f ? x0 : 0.f, r1 != 0.f ? x1 : 0.f);
+  }
+  const float4 f = *reinterpret_cast<const float4*>(t.p + q.k);
+  const float y[4] = {f.x, f.y, f.z, f.w};
+  by_colour(q, y, p);
+  p[0] = add2(p[0], d[0]); p[1] = add2(p[1], d[1]);
+}
+// a ring cell's plan, from the coefficients and level sizes alone: bits 0-10 box index, 11-19 its
+// coarse cell in the coarse box, 20-21 and 22-23 the steps to the other coarse column and row plus
+// one, 24 open
 static_assert(MGF_BW * MGF_BH <= 2048 && MGF_CBW * MGF_CBH <= 512, "plan fields");
-__device__ __forceinline__ void prolong_plan(const Tile& t, const LevelDesc& L, const LevelDesc& C, int x0, int y0,
-                                             int cx, int cy, uint32_t (&pl)[PR_N]) {
-  #pragma unroll
-  for (int m = 0; m < PR_N; m++) {
-    const int e = threadIdx.x + 256 * m;
-    const int i = x0 - MGF_H + e % PR_W, j = y0 - MGF_H + e / PR_W;
-    pl[m] = 0u;
-    if (e >= PR_W * PR_H || i < 0 || i >= L.nx || j < 0 || j >= L.ny) continue;
-    const int I = i / 2, J = j / 2;
-    const int dI = min(max(I + ((i & 1) == 1 ? 1 : -1), 0), C.nx - 1) - I;
-    const int dJ = min(max(J + ((j & 1) == 1 ? 1 : -1), 0), C.ny - 1) - J;
-    const int a = (J - cy) * MGF_CBW + I - cx;
-    pl[m] = (uint32_t)t.c(i, j) | (uint32_t)a << 11 | (uint32_t)(dI + 1) << 20 | (uint32_t)(dJ + 1) << 22 |
-            (diag_s(t, L.nx, L.ny, i, j) > 0.f ? 1u << 24 : 0u) | 1u << 25;
-  }
+__device__ __forceinline__ uint32_t ring_plan(const Tile& t, const LevelDesc& L, const LevelDesc& C, int cx, int cy) {
+  if (threadIdx.x >= RING_N) return 0u;
+  int br, bc;
+  ring_cell(threadIdx.x, br, bc);
+  const int i = t.sx + bc, j = t.sy + br;
+  const uint32_t k = br * MGF_BW + bc;
+  if (i < 0 || i >= L.nx || j < 0 || j >= L.ny) return k;
+  const int I = i / 2, J = j / 2;
+  const int dI = min(max(I + ((i & 1) == 1 ? 1 : -1), 0), C.nx - 1) - I;
+  const int dJ = min(max(J + ((j & 1) == 1 ? 1 : -1), 0), C.ny - 1) - J;
+  return k | (uint32_t)((J - cy) * MGF_CBW + I - cx) << 11 | (uint32_t)(dI + 1) << 20 | (uint32_t)(dJ + 1) << 22 |
+         (diag_s(t, L.nx, L.ny, i, j) > 0.f ? 1u << 24 : 0u);
 }
-// the same additions computed in one pass after the coarse box has landed (several scenes: the
-// plan would only add instructions after the wait)
-__device__ __forceinline__ void prolong_direct(const Tile& t, const LevelDesc& L, const LevelDesc& C, int x0, int y0,
-                                               int cx, int cy, const float* scp) {
-  for (int e = threadIdx.x; e < PR_W * PR_H; e += 256) {
-    const int i = x0 - MGF_H + e % PR_W, j = y0 - MGF_H + e / PR_W;
-    if (i < 0 || i >= L.nx || j < 0 || j >= L.ny) continue;
-    const int I = i / 2, J = j / 2;
-    const int I2 = min(max(I + ((i & 1) == 1 ? 1 : -1), 0), C.nx - 1);
-    const int J2 = min(max(J + ((j & 1) == 1 ? 1 : -1), 0), C.ny - 1);
-    const int r0 = (J - cy) * MGF_CBW, r1 = (J2 - cy) * MGF_CBW;
-    const float c_ = 0.5625f * scp[r0 + I - cx] + 0.1875f * (scp[r0 + I2 - cx] + scp[r1 + I - cx]) +
-                     0.0625f * scp[r1 + I2 - cx];
-    t.p[t.c(i, j)] += diag_s(t, L.nx, L.ny, i, j) > 0.f ? c_ : 0.f;
+__device__ __forceinline__ void prolong_ring(const Tile& t, float* sp, const float* scp, uint32_t pl) {
+  if (threadIdx.x >= RING_N) return;
+  const int k = pl & 2047, br = k / MGF_BW, bc = k - br * MGF_BW;
+  float c = 0.f;
+  if (pl & (1u << 24)) {
+    const int a = (pl >> 11) & 511, dI = (int)((pl >> 20) & 3) - 1, dJ = ((int)((pl >> 22) & 3) - 1) * MGF_CBW;
+    c = 0.5625f * scp[a] + 0.1875f * (scp[a + dI] + scp[a + dJ]) + 0.0625f * scp[a + dI + dJ];
   }
+  sp[sp_at(br, bc, t.sx, t.sy)] = t.p[k] + c;
 }
-__device__ __forceinline__ void prolong_apply(const Tile& t, const float* scp, const uint32_t (&pl)[PR_N]) {
-  #pragma unroll
-  for (int m = 0; m < PR_N; m++) {
-    const uint32_t q = pl[m];
-    if (!(q & (1u << 25))) continue;
-    const int a = (q >> 11) & 511, dI = (int)((q >> 20) & 3) - 1, dJ = ((int)((q >> 22) & 3) - 1) * MGF_CBW;
-    const float c_ = 0.5625f * scp[a] + 0.1875f * (scp[a + dI] + scp[a + dJ]) + 0.0625f * scp[a + dI + dJ];
-    t.p[q & 2047] += (q & (1u << 24)) ? c_ : 0.f;
-  }
+// four values of a level row from column i on (those inside the level)
+__device__ __forceinline__ void store4(float* row, int i, int nx, float4 v) {
+  if (i + 3 < nx) { *reinterpret_cast<float4*>(row + i) = v; return; }
+  if (i < nx) row[i] = v.x;
+  if (i + 1 < nx) row[i + 1] = v.y;
+  if (i + 2 < nx) row[i + 2] = v.z;
 }
 
 // Fused Krylov mode on level 0 (all scenes' coarse blocks start below it). The update of
@@ -298,60 +388,43 @@ __device__ __forceinline__ void prolong_apply(const Tile& t, const float* scp, c
 // partials; k_pcg_decide (one CTA per scene, the next kernel) sums them, forms the cycle's
 // alpha and beta, and ||r_c||^2 = r.r - 2 alpha r.q_c + alpha^2 q_c.q_c (q_c = Lz + beta q)
 // for the loop decision.
-// This thread's share of the down kernel's update: up to 4 cells of pass 1's region and
-// 2 tile cells, with their stored values loaded right after the wait.
-struct PcgDown {
-  double r[4], q[4], lz[4], dA[2], p64[2];
-  float z[2];
-};
-__device__ __forceinline__ void pcg_down_load(const SceneDesc& S, const LevelDesc& L, int x0, int y0, PcgDown& u) {
-  constexpr int N1 = SM_W1 * SM_H1;
-  #pragma unroll
-  for (int m = 0; m < 4; m++) {
-    const int e = threadIdx.x + 256 * m;
-    const int i = x0 - MGF_H + 1 + e % SM_W1, j = y0 - MGF_H + 1 + e / SM_W1;
-    if (e < N1 && i >= 0 && i < L.nx && j >= 0 && j < L.ny) {
-      const int k = j * L.nx + i;
-      u.r[m] = __ldcg(S.r64 + k); u.q[m] = __ldcg(S.q64 + k); u.lz[m] = __ldcg(S.dB + k);
+// Two consecutive doubles of a dense FP64 row (nx is even on a level with one below it, and the
+// column too: 16-byte aligned)
+__device__ __forceinline__ double2 ldcg2(const double* p) { return __ldcg(reinterpret_cast<const double2*>(p)); }
+// the item's new rhs0 in column order, from its stored r, q, Lz
+__device__ __forceinline__ float4 pcg_rhs(const SceneDesc& S, const LevelDesc& L, const Item& q, const PcgPrev& pv) {
+  float v[4] = {0.f, 0.f, 0.f, 0.f};
+  if (q.on && (unsigned)q.j < (unsigned)L.ny) {
+    const bool first = pv.cycles == 1;
+    #pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const int i = q.base + 2 * h;
+      if (i < 0 || i >= L.nx) continue;
+      const size_t k = (size_t)q.j * L.nx + i;
+      const double2 r = ldcg2(S.r64 + k), qq = ldcg2(S.q64 + k), lz = ldcg2(S.dB + k);
+      v[2 * h] = (float)(r.x - pv.alpha * (first ? lz.x : lz.x + pv.beta * qq.x));
+      v[2 * h + 1] = (float)(r.y - pv.alpha * (first ? lz.y : lz.y + pv.beta * qq.y));
     }
   }
-  #pragma unroll
-  for (int m = 0; m < 2; m++) {
-    const int e = threadIdx.x + 256 * m;
-    const int i = x0 + e % MGF_TX, j = y0 + e / MGF_TX;
-    if (i < L.nx && j < L.ny) {
-      u.dA[m] = __ldcg(S.dA + j * L.nx + i); u.p64[m] = __ldcg(S.p64 + j * L.nx + i);
-      u.z[m] = __ldcg(L.p + j * L.pc + i);
-    }
-  }
+  return make_float4(v[0], v[1], v[2], v[3]);
 }
-// after the state barrier: p = 0 on the whole box, rhs0 on pass 1's region, d and p64 on the
-// tile (rhs0 of the tile to global for the up kernel's staging once the block has synced)
-__device__ __forceinline__ void pcg_down_apply(const SceneDesc& S, const LevelDesc& L, const Tile& t, int x0, int y0,
-                                               const PcgPrev& pv, const PcgDown& u) {
-  constexpr int N1 = SM_W1 * SM_H1;
+// d and p64 of the item's cells (z: the last cycle's p)
+__device__ __forceinline__ void pcg_dir(const SceneDesc& S, const LevelDesc& L, const Item& q, const PcgPrev& pv) {
+  if (q.j >= L.ny) return;
   const bool first = pv.cycles == 1;
-  for (int e = threadIdx.x; e < MGF_BW * MGF_BH; e += 256) t.p[e] = 0.f;
   #pragma unroll
-  for (int m = 0; m < 4; m++) {
-    const int e = threadIdx.x + 256 * m;
-    const int i = x0 - MGF_H + 1 + e % SM_W1, j = y0 - MGF_H + 1 + e / SM_W1;
-    if (e < N1 && i >= 0 && i < L.nx && j >= 0 && j < L.ny) {
-      const double q = first ? u.lz[m] : u.lz[m] + pv.beta * u.q[m];
-      const double r = u.r[m] - pv.alpha * q;
-      t.rhs[t.c(i, j)] = (float)r;
-    }
-  }
-  #pragma unroll
-  for (int m = 0; m < 2; m++) {
-    const int e = threadIdx.x + 256 * m;
-    const int i = x0 + e % MGF_TX, j = y0 + e / MGF_TX;
-    if (i < L.nx && j < L.ny) {
-      const double z = (double)u.z[m];
-      const double d = first ? z : z + pv.beta * u.dA[m];
-      S.dA[j * L.nx + i] = d;
-      S.p64[j * L.nx + i] = u.p64[m] + pv.alpha * d;
-    }
+  for (int h = 0; h < 2; h++) {
+    const int i = q.base + 2 * h;
+    if (i >= L.nx) continue;
+    const size_t k = (size_t)q.j * L.nx + i;
+    const float2 z = __ldcg(reinterpret_cast<const float2*>(L.p + (size_t)q.j * L.pc + i));
+    double2 d = ldcg2(S.dA + k), p = ldcg2(S.p64 + k);
+    d.x = first ? (double)z.x : (double)z.x + pv.beta * d.x;
+    d.y = first ? (double)z.y : (double)z.y + pv.beta * d.y;
+    p.x += pv.alpha * d.x;
+    p.y += pv.alpha * d.y;
+    *reinterpret_cast<double2*>(S.dA + k) = d;
+    *reinterpret_cast<double2*>(S.p64 + k) = p;
   }
 }
 
@@ -360,28 +433,26 @@ __device__ __forceinline__ void pcg_down_apply(const SceneDesc& S, const LevelDe
 // ------------------------------------------------------------------ down: 4 passes + restrict
 // PCG: the fused Krylov update on level 0 (above)
 // ONE: compiled for an engine of one scene (nscenes == 1), whose flag only ends the loop
-// MINB: resident CTAs per SM the registers are sized for (3; 2 for a level-0 Krylov kernel whose
-// tiles fit in one wave at two per SM: no spill)
+// MINB: resident CTAs per SM the registers are sized for
+// MEASURED_LEVEL
 template <int TX, int TY, bool PCG, bool ONE, int MINB = 3>
-// three CTAs per SM (at most 85 registers a thread; 44 bytes of spill in the fused Krylov
-// variant): 512x768's 768 level-0 tiles run in two waves instead of three (measured: -5% per
-// Krylov cycle at 512x768). Four for the plain variants (62 registers) was measured 3-4% slower
-// per step at 256x384 and 512x768 and no faster for the batch.
 __global__ void __launch_bounds__(256, MINB) k_mg_down(const SceneDesc* __restrict__ scenes, int nscenes, const Work* __restrict__ work,
-                                                 int level, SolveCtl* ctl, int count_iter) {
+                                                 int level, SolveCtl* ctl, int count_iter, f2 nz) {
   static_assert(TX == MGF_TX && TY == MGF_TY, "the tensor-map boxes are built for the MGF tile");
-  __shared__ __align__(128) float sp[MGF_BH * MGF_BW];
+  __shared__ __align__(128) float bp[MGF_BH * MGF_BW];
   __shared__ __align__(128) float srhs[MGF_BH * MGF_BW];
   __shared__ __align__(128) float sax[MGF_BH * MGF_BW];
   __shared__ __align__(128) float say[(MGF_BH + 1) * MGF_BW];
-  __shared__ float sr[TY * TX];
+  __shared__ __align__(16) float sp[SP_N];
+  __shared__ __align__(16) float sr[TY / 2 * TX];   // odd rows' residuals
   __shared__ __align__(8) uint64_t bar[2];
   const Work w = work[blockIdx.x];
   const SceneDesc& S = scenes[w.scene];
   pdl_trigger();
   const LevelDesc L = S.lev[level], C = S.lev[level + 1];
   const int x0 = w.tx * TX, y0 = w.ty * TY;
-  const Tile t{sp, srhs, sax, say, x0 - MGF_SX, y0 - MGF_H};
+  const Tile t{bp, srhs, sax, say, x0 - MGF_SX, y0 - MGF_H};
+  const Item q = item_of(x0, y0);
   const bool on = S.enabled;   // host-written, constant during the step
   SolveState* ss = S.solve;
   // one scene: its flag only ends the loop, so the tile is requested before it is read;
@@ -396,17 +467,17 @@ __global__ void __launch_bounds__(256, MINB) k_mg_down(const SceneDesc* __restri
       prefetch_state_maps(S, level, TM_P, false);
     }
   }
-  // below level 0 the level's p is zero on entry (the restriction above zeroes it): with one
-  // scene its box is zero-filled before the wait instead of copied after it
-  const bool pz = spec && level > 0;
-  if (pz)
-    for (int e = threadIdx.x; e < MGF_BW * MGF_BH; e += 256) t.p[e] = 0.f;
+  // below level 0 the level's p is zero on entry (the restriction above zeroes it)
+  const bool pz = level > 0;
+  f2 p[2];
+  zero_sp(sp, p);
   __syncthreads();
   const bool idle = on && spec && s_idle;
   // one scene: the stencils, which depend on the coefficients alone, are built before the wait
-  TCell c[2][2];
+  Sten c;
+  c.nz = nz;
   bool ok = true;
-  if (on && spec && !idle && (ok = tile_wait(&bar[0], ctl))) tile_stencils(t, L, x0, y0, 0, c);
+  if (on && spec && !idle && (ok = tile_wait(&bar[0], ctl))) item_stencils(t, L, q, c);
   pdl_wait();
   if (count_iter && blockIdx.x == 0 && threadIdx.x == 0) loop_count(ctl);
   if (!on || !ok || idle) return;
@@ -416,55 +487,69 @@ __global__ void __launch_bounds__(256, MINB) k_mg_down(const SceneDesc* __restri
     __syncthreads();
   }
   PcgPrev pv{};
-  PcgDown u;
-  if (PCG) {
-    pv = pcg_load(ss);
-    pcg_down_load(S, L, x0, y0, u);
-  }
+  if (PCG) pv = pcg_load(ss);
   const bool live = *(volatile int*)&ss->active != 0;
   const bool upd = PCG && pv.cycles >= 1;   // an update of the previous cycle is pending
   stage_state(S, level, TM_P, t, !upd, nullptr, 0, 0, bar, !pz);
-  if (!(spec ? tile_wait(&bar[1], ctl) : tile_wait2(bar, ctl, [&] { tile_stencils(t, L, x0, y0, 0, c); })) || !live)
+  float4 rv = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (PCG && upd && live) rv = pcg_rhs(S, L, q, pv);
+  if (!(spec ? tile_wait(&bar[1], ctl) : tile_wait2(bar, ctl, [&] { item_stencils(t, L, q, c); })) || !live)
     return;
+  const bool mine = in_tile(q, x0, y0);
+  f2 rhs[2];
   if (upd) {
-    pcg_down_apply(S, L, t, x0, y0, pv, u);
-    __syncthreads();
-    for (int e = threadIdx.x; e < TX * TY; e += blockDim.x) {
-      const int i = x0 + e % TX, j = y0 + e / TX;
-      if (i < L.nx && j < L.ny) L.rhs[j * L.pc + i] = t.rhs[t.c(i, j)];
-    }
+    // rhs0 of the tile also to global, for the up kernel's staging
+    if (mine && q.j < L.ny) store4(L.rhs + (size_t)q.j * L.pc, q.base, L.nx, rv);
+  } else if (q.on) {
+    rv = *reinterpret_cast<const float4*>(t.rhs + q.k);
   }
-  tile_passes(t, L, 0, c);   // colours 0, 1, 0, 1 (js/fluid.js:298-301)
-  // residual of the tile cells (pressure.wgsl:96-101) from the slots' stencils (every tile cell
-  // of the level is a slot of some thread); the quotient by h2 from RN(1/h2), the IEEE one
-  const float rh2 = __frcp_rn(L.h2);
-  #pragma unroll
-  for (int col = 0; col < 2; col++)
+  item_rhs(q, L.h2, rv, c, rhs);
+  if (!upd && !pz) {
+    stage_sp(t, sp, q, p);
+    __syncthreads();
+  }
+  item_passes(sp, q, c, 0, p);   // colours 0, 1, 0, 1 (js/fluid.js:298-301)
+  // residual of the tile cells (pressure.wgsl:96-101) from the items' stencils; the quotient by h2
+  // from RN(1/h2), the IEEE one; then the restriction (pressure.wgsl:104-113): the even rows' items
+  // add the odd rows' residuals to their own
+  float4 res = make_float4(0.f, 0.f, 0.f, 0.f);
+  const int tr = q.r - (MGF_H - 1), ti = q.base - x0;   // tile row and column
+  if (mine) {
+    const float h = L.h2, rh = __frcp_rn(h);
+    const f2 nh = pk(-h, -h), rh2 = pk(rh, rh), m1 = pk(-1.f, -1.f);
+    f2 r[2];
     #pragma unroll
-    for (int m = 0; m < 2; m++) {
-      const TCell& q = c[col][m];
-      if (!(q.fl & 1)) continue;
-      const int bj = q.kp / MGF_BW, bi = q.kp - bj * MGF_BW;   // box row and column
-      const float off = tcell_off(t, q);
-      sr[(bj - MGF_H) * TX + (bi - MGF_SX)] =
-          q.diag <= 0.f ? 0.f : t.rhs[q.kp] - mgc::div_by_rcp(off - q.diag * t.p[q.kp], L.h2, rh2);
+    for (int col = 0; col < 2; col++) {
+      const f2 x = add2(item_off(sp, q, c, col, p[1 - col]), mul2(c.nd[col], p[col], c.nz));
+      r[col] = fma2(quot2(x, nh, rh2, c.nz), m1, rhs[col]);
+      float r0, r1, d0, d1;
+      upk(c.rc[col], d0, d1);
+      upk(r[col], r0, r1);
+      r[col] = pk(d0 != 0.f ? r0 : 0.f, d1 != 0.f ? r1 : 0.f);
     }
-  // the smoothed p
-  for (int e = threadIdx.x; e < TX * TY; e += blockDim.x) {
-    const int i = x0 + e % TX, j = y0 + e / TX;
-    if (i < L.nx && j < L.ny) L.pb[j * L.pc + i] = t.p[t.c(i, j)];
+    res = in_order(q, r);
+    if (tr & 1) *reinterpret_cast<float4*>(sr + (tr >> 1) * TX + ti) = res;
+    if (q.j < L.ny) store4(L.pb + (size_t)q.j * L.pc, q.base, L.nx, in_order(q, p));   // the smoothed p
   }
   __syncthreads();
-  // restriction (pressure.wgsl:104-113)
-  constexpr int CX = TX / 2, CY = TY / 2;
-  for (int e = threadIdx.x; e < CX * CY; e += blockDim.x) {
-    const int a = e % CX, b = e / CX, I = x0 / 2 + a, J = y0 / 2 + b;
-    if (I >= C.nx || J >= C.ny) continue;
-    const float r = sr[(2 * b) * TX + 2 * a] + sr[(2 * b) * TX + 2 * a + 1] + sr[(2 * b + 1) * TX + 2 * a] +
-                    sr[(2 * b + 1) * TX + 2 * a + 1];
-    C.rhs[J * C.pc + I] = 0.25f * r;
-    C.p[J * C.pc + I] = 0.f;
+  if (mine && !(tr & 1)) {
+    const float4 o = *reinterpret_cast<const float4*>(sr + (tr >> 1) * TX + ti);
+    const int I = q.base / 2, J = q.j / 2;
+    if (J < C.ny) {
+      const float v0 = 0.25f * (res.x + res.y + o.x + o.y), v1 = 0.25f * (res.z + res.w + o.z + o.w);
+      float* cr = C.rhs + (size_t)J * C.pc + I;
+      float* cp = C.p + (size_t)J * C.pc + I;
+      if (I + 1 < C.nx) {
+        *reinterpret_cast<float2*>(cr) = make_float2(v0, v1);
+        *reinterpret_cast<float2*>(cp) = make_float2(0.f, 0.f);
+      } else if (I < C.nx) {
+        *cr = v0;
+        *cp = 0.f;
+      }
+    }
   }
+  // the pending direction and pressure (read and written by this item alone)
+  if (PCG && upd && mine) pcg_dir(S, L, q, pv);
 }
 
 // ------------------------------------------------------------------ up: prolong + 4 passes (+ level-0 tail)
@@ -474,16 +559,17 @@ __global__ void __launch_bounds__(256, MINB) k_mg_down(const SceneDesc* __restri
 // instance per tail (levels below 0: tail 0)
 template <int TX, int TY, int TAIL, bool ONE, int MINB = 3>   // ONE, MINB: as in k_mg_down
 __global__ void __launch_bounds__(256, MINB) k_mg_up(const SceneDesc* __restrict__ scenes, int nscenes, const Work* __restrict__ work,
-                                               int level, SolveCtl* ctl) {
+                                               int level, SolveCtl* ctl, f2 nz) {
   static_assert(TX == MGF_TX && TY == MGF_TY, "the tensor-map boxes are built for the MGF tile");
   static_assert(TAIL >= 0 && TAIL <= 4, "tails 0-4");
   constexpr bool KRY = TAIL == 4;
   constexpr int tail = TAIL;
-  __shared__ __align__(128) float sp[MGF_BH * MGF_BW];
+  __shared__ __align__(128) float bp[MGF_BH * MGF_BW];
   __shared__ __align__(128) float srhs[MGF_BH * MGF_BW];
   __shared__ __align__(128) float sax[MGF_BH * MGF_BW];
   __shared__ __align__(128) float say[(MGF_BH + 1) * MGF_BW];
   __shared__ __align__(128) float scp[MGF_CBH * MGF_CBW];
+  __shared__ __align__(16) float sp[SP_N];
   __shared__ double red[32];
   __shared__ __align__(8) uint64_t bar[2];
   const Work w = work[blockIdx.x];
@@ -491,7 +577,8 @@ __global__ void __launch_bounds__(256, MINB) k_mg_up(const SceneDesc* __restrict
   pdl_trigger();
   const LevelDesc L = S.lev[level], C = S.lev[level + 1];
   const int x0 = w.tx * TX, y0 = w.ty * TY;
-  const Tile t{sp, srhs, sax, say, x0 - MGF_SX, y0 - MGF_H};
+  const Tile t{bp, srhs, sax, say, x0 - MGF_SX, y0 - MGF_H};
+  const Item q = item_of(x0, y0);
   // coarse p under the region: columns x0/2-4 .. x0/2+TX/2+3, rows y0/2-4 .. y0/2+TY/2+3
   const int cx = x0 / 2 - 8, cy = y0 / 2 - 4;
   const bool on = S.enabled;   // host-written, constant during the step
@@ -507,17 +594,19 @@ __global__ void __launch_bounds__(256, MINB) k_mg_up(const SceneDesc* __restrict
     }
   }
   __shared__ double s_rh2;   // the FP64 operator's 1 / h2 (tails 3 and 4)
-  if (threadIdx.x == 0) s_rh2 = 1.0 / (double)L.h2;
+  if ((tail == 3 || tail == 4) && threadIdx.x == 0) s_rh2 = 1.0 / (double)L.h2;
   __syncthreads();
   const bool idle = on && spec && s_idle;
-  const double rh2 = s_rh2;
-  TCell c[2][2];
-  uint32_t pl[PR_N];
+  const double rh2 = tail == 3 || tail == 4 ? s_rh2 : 0.0;
+  Sten c;
+  c.nz = nz;
+  uint32_t pl = 0u;
   bool ok = true;
-  if (on && spec && !idle && (ok = tile_wait(&bar[0], ctl))) {
-    tile_stencils(t, L, x0, y0, 1, c);
-    prolong_plan(t, L, C, x0, y0, cx, cy, pl);
-  }
+  auto prepare = [&] {
+    item_stencils(t, L, q, c);
+    pl = ring_plan(t, L, C, cx, cy);
+  };
+  if (on && spec && !idle && (ok = tile_wait(&bar[0], ctl))) prepare();
   pdl_wait();
   if (!on || !ok || idle) return;
   if (!spec) {
@@ -542,15 +631,23 @@ __global__ void __launch_bounds__(256, MINB) k_mg_up(const SceneDesc* __restrict
       }
     }
   }
-  if (!(spec ? tile_wait(&bar[1], ctl) : tile_wait2(bar, ctl, [&] { tile_stencils(t, L, x0, y0, 1, c); })) || !live)
+  if (!(spec ? tile_wait(&bar[1], ctl) : tile_wait2(bar, ctl, prepare)) || !live)
     return;
   // prolongation (pressure.wgsl:116-129) on the whole region
-  if (spec)
-    prolong_apply(t, scp, pl);
-  else
-    prolong_direct(t, L, C, x0, y0, cx, cy, scp);
+  f2 p[2] = {0ull, 0ull};
+  if (q.on) {
+    item_rhs(q, L.h2, *reinterpret_cast<const float4*>(t.rhs + q.k), c);
+    prolong_item(t, C, q, c, cx, cy, scp, p);
+    put_item(sp, q, p);
+  }
+  prolong_ring(t, sp, scp, pl);
   __syncthreads();
-  tile_passes(t, L, 1, c);   // colours 1, 0, 1, 0 (js/fluid.js:307-310)
+  item_passes(sp, q, c, 1, p);   // colours 1, 0, 1, 0 (js/fluid.js:307-310)
+  if (in_tile(q, x0, y0) && q.j < L.ny) store4(L.p + (size_t)q.j * L.pc, q.base, L.nx, in_order(q, p));
+  if (tail == 0) return;
+  // the tails read the tile and its ring from the box again
+  if (q.on) *reinterpret_cast<float4*>(t.p + q.k) = in_order(q, p);
+  __syncthreads();
   if (KRY) {
     // the pending r, q update (cycles >= 1), then r.z, q.z, z.Lz and the recurrence's r.r,
     // r.Lz, r.q, Lz.Lz, Lz.q, q.q on the tile
@@ -562,20 +659,19 @@ __global__ void __launch_bounds__(256, MINB) k_mg_up(const SceneDesc* __restrict
       const int i = x0 + e % TX, j = y0 + e / TX;
       if (i >= L.nx || j >= L.ny) continue;
       const int k = t.c(i, j), kk = j * L.nx + i;
-      L.p[j * L.pc + i] = t.p[k];
-      double r = r0[m], q = q0[m];
+      double r = r0[m], qv = q0[m];
       if (upd) {
-        q = first ? lz0[m] : lz0[m] + pv.beta * q;
-        r = r - pv.alpha * q;
-        S.q64[kk] = q;
+        qv = first ? lz0[m] : lz0[m] + pv.beta * qv;
+        r = r - pv.alpha * qv;
+        S.q64[kk] = qv;
         S.r64[kk] = r;
       }
       const double z = (double)t.p[k];
       const double lz = lap_tile64(t, L, i, j, rh2);
       S.dB[kk] = lz;
-      v[0] = __fma_rn(r, z, v[0]); v[1] = __fma_rn(q, z, v[1]); v[2] = __fma_rn(z, lz, v[2]);
-      v[3] = __fma_rn(r, r, v[3]); v[4] = __fma_rn(r, lz, v[4]); v[5] = __fma_rn(r, q, v[5]);
-      v[6] = __fma_rn(lz, lz, v[6]); v[7] = __fma_rn(lz, q, v[7]); v[8] = __fma_rn(q, q, v[8]);
+      v[0] = __fma_rn(r, z, v[0]); v[1] = __fma_rn(qv, z, v[1]); v[2] = __fma_rn(z, lz, v[2]);
+      v[3] = __fma_rn(r, r, v[3]); v[4] = __fma_rn(r, lz, v[4]); v[5] = __fma_rn(r, qv, v[5]);
+      v[6] = __fma_rn(lz, lz, v[6]); v[7] = __fma_rn(lz, qv, v[7]); v[8] = __fma_rn(qv, qv, v[8]);
     }
     // the tile's nine partials, quantity-major (part[m * nt_up0 + tile]); k_pcg_decide sums
     // them once this kernel has completed (no arrival, no fence in these CTAs)
@@ -591,7 +687,6 @@ __global__ void __launch_bounds__(256, MINB) k_mg_up(const SceneDesc* __restrict
     const int i = x0 + e % TX, j = y0 + e / TX;
     if (i >= L.nx || j >= L.ny) continue;
     const int k = t.c(i, j);
-    L.p[j * L.pc + i] = t.p[k];
     if (tail == 1) {
       float off, diag; stencil_s(t, L.nx, L.ny, i, j, off, diag);
       const double r = diag <= 0.f ? 0.0 : (double)(t.rhs[k] - (off - diag * t.p[k]) / L.h2);
@@ -618,9 +713,9 @@ __global__ void __launch_bounds__(256, MINB) k_mg_up(const SceneDesc* __restrict
     return;
   }
   if (tail != 1) return;
-  const double bp = block_sum(part, red);
+  const double bpart = block_sum(part, red);
   double total = 0.0;
-  if (scene_reduce(S, w.tile, S.nt_up0, bp, red, &total) && threadIdx.x == 0) solve_decide(ctl, ss, total, true);
+  if (scene_reduce(S, w.tile, S.nt_up0, bpart, red, &total) && threadIdx.x == 0) solve_decide(ctl, ss, total, true);
 }
 
 // ------------------------------------------------------------------ fused Krylov mode: the loop decision
@@ -1394,7 +1489,8 @@ size_t coarse_smem_bytes(const int* lnx, const int* lny, int lc, int nlev) {
   return f * 4;
 }
 
-using UpKernel = void (*)(const SceneDesc*, int, const Work*, int, SolveCtl*);
+using UpKernel = void (*)(const SceneDesc*, int, const Work*, int, SolveCtl*, f2);
+constexpr f2 kNegZero2 = 0x8000000080000000ull;
 template <bool ONE>
 static UpKernel up_kernel(int tail) {
   switch (tail) {
@@ -1423,7 +1519,7 @@ void launch_mg_down(const SceneDesc* scenes, int nscenes, const Work* work, int 
                                                        : k_mg_down<MGF_TX, MGF_TY, true, true>)
                             : k_mg_down<MGF_TX, MGF_TY, false, true>)
                      : (pcg ? k_mg_down<MGF_TX, MGF_TY, true, false> : k_mg_down<MGF_TX, MGF_TY, false, false>);
-  launch_pdl(pdl && pdl_enabled(), k, dim3(ntiles), dim3(256), 0, st, scenes, nscenes, work, level, ctl, count_iter);
+  launch_pdl(pdl && pdl_enabled(), k, dim3(ntiles), dim3(256), 0, st, scenes, nscenes, work, level, ctl, count_iter, kNegZero2);
 }
 void launch_mg_up(const SceneDesc* scenes, int nscenes, const Work* work, int ntiles, int level, int tail, SolveCtl* ctl,
                   cudaStream_t st) {
@@ -1431,7 +1527,7 @@ void launch_mg_up(const SceneDesc* scenes, int nscenes, const Work* work, int nt
   const UpKernel k = nscenes != 1 ? up_kernel<false>(tail)
                      : tail == 4 && one_wave_at_two(ntiles) ? k_mg_up<MGF_TX, MGF_TY, 4, true, 2>
                                                             : up_kernel<true>(tail);
-  launch_pdl(pdl_enabled(), k, dim3(ntiles), dim3(256), 0, st, scenes, nscenes, work, level, ctl);
+  launch_pdl(pdl_enabled(), k, dim3(ntiles), dim3(256), 0, st, scenes, nscenes, work, level, ctl, kNegZero2);
 }
 void launch_pcg_decide(const SceneDesc* scenes, int nscenes, SolveCtl* ctl, cudaStream_t st) {
   if (nscenes > 0) launch_pdl(pdl_enabled(), k_pcg_decide, dim3(nscenes), dim3(256), 0, st, scenes, ctl);
