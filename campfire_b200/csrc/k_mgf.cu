@@ -433,9 +433,15 @@ __device__ __forceinline__ void pcg_dir(const SceneDesc& S, const LevelDesc& L, 
 // ------------------------------------------------------------------ down: 4 passes + restrict
 // PCG: the fused Krylov update on level 0 (above)
 // ONE: compiled for an engine of one scene (nscenes == 1), whose flag only ends the loop
-// MINB: resident CTAs per SM the registers are sized for
-// MEASURED_LEVEL
-template <int TX, int TY, bool PCG, bool ONE, int MINB = 3>
+// MINB: resident CTAs per SM the registers are sized for: three for one scene (four cost 512x768
+// 3.5% per step), two for its level-0 Krylov kernels where the tiles fit in one wave at two per SM
+// (256x384: three cost 2%), four for several scenes (64 uneven ones: three cost 5%, five 7%)
+// Bound by instruction issue where the tiles fill the GPU and by the chain copy - passes - stores
+// where they do not. With each thread's two cells of each colour a stride apart and unpacked
+// arithmetic (scalar loads of four neighbours and four coefficients per cell, the FP64 update and
+// the stencils in different maps) a step took 814 us at 512x768, 288 at 256x384, 95.4 at 224x320
+// and 4655 for the 64-scene batch; with items 741, 270, 91.9 and 3903.
+template <int TX, int TY, bool PCG, bool ONE, int MINB = ONE ? 3 : 4>
 __global__ void __launch_bounds__(256, MINB) k_mg_down(const SceneDesc* __restrict__ scenes, int nscenes, const Work* __restrict__ work,
                                                  int level, SolveCtl* ctl, int count_iter, f2 nz) {
   static_assert(TX == MGF_TX && TY == MGF_TY, "the tensor-map boxes are built for the MGF tile");
@@ -557,7 +563,7 @@ __global__ void __launch_bounds__(256, MINB) k_mg_down(const SceneDesc* __restri
 // 3 r.z, q.z, z.Lz -> the direction update (Krylov FP64 mode), 4 the same in the fused Krylov
 // mode (the pending r, q update first; the loop decision from the recurrence for ||r||); one
 // instance per tail (levels below 0: tail 0)
-template <int TX, int TY, int TAIL, bool ONE, int MINB = 3>   // ONE, MINB: as in k_mg_down
+template <int TX, int TY, int TAIL, bool ONE, int MINB = ONE ? 3 : 4>   // ONE, MINB: as in k_mg_down
 __global__ void __launch_bounds__(256, MINB) k_mg_up(const SceneDesc* __restrict__ scenes, int nscenes, const Work* __restrict__ work,
                                                int level, SolveCtl* ctl, f2 nz) {
   static_assert(TX == MGF_TX && TY == MGF_TY, "the tensor-map boxes are built for the MGF tile");
