@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include <cstddef>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -252,11 +253,13 @@ class Engine {
   // cfg_write_params reads it once that event has passed instead of reading the descriptor back
   // (dt_from_step_: no descriptor upload since that step)
   float *h_dt_pinned_ = nullptr, *d_dtv_ = nullptr;
+  static constexpr size_t kIoBytes = 256 * 1024;   // staging area of reads, pinned and mapped
+  char *h_io_ = nullptr, *d_io_ = nullptr;
+  std::mutex io_mu_;                               // the scenes of a batch share the staging area
   cudaEvent_t ev_dt_ = nullptr;
   bool dt_from_step_ = false;
   double* d_dxd_ = nullptr;
   double* d_alpha_ = nullptr;
-  double* d_scratch_ = nullptr;   // small FP64 outputs (budgets, norms)
   float* d_rwood_ = nullptr;      // the renderer's wood buffer (MAX_PIECES x 12 floats)
   float* d_image_ = nullptr;      // the renderer's output image
   size_t image_bytes_ = 0;

@@ -515,6 +515,16 @@ __global__ void k_readback(uint32_t* __restrict__ src, uint32_t* __restrict__ ho
   __threadfence_system();
 }
 
+// One word per thread and round; a row's words stay together, so both sides are coalesced.
+__global__ void __launch_bounds__(256) k_pack(uint32_t* __restrict__ dst, const char* __restrict__ src, size_t pitch, int w, int h) {
+  for (int j = blockIdx.y; j < h; j += gridDim.y)
+    for (int i = blockIdx.x * 256 + threadIdx.x; i < w; i += gridDim.x * 256)
+      dst[(size_t)j * w + i] = __ldg(reinterpret_cast<const uint32_t*>(src + (size_t)j * pitch) + i);
+}
+void launch_pack(uint32_t* dst, const void* src, size_t pitch, int w, int h, cudaStream_t st) {
+  if (w > 0 && h > 0)
+    k_pack<<<dim3((w + 255) / 256, h < 2048 ? h : 2048), 256, 0, st>>>(dst, static_cast<const char*>(src), pitch, w, h);
+}
 void launch_write_params(uint32_t* dst, const ParamWords& b, int skip, int s0, int s1, cudaStream_t st) {
   k_write_params<<<1, 64, 0, st>>>(dst, b, skip, s0, s1);
 }

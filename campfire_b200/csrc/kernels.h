@@ -104,6 +104,8 @@ void launch_write_params(uint32_t* dst, const ParamWords& b, int skip, int s0, i
 void launch_write_pieces(float* dst, const PieceFloats& b, cudaStream_t st);
 // nwords words of src to mapped pinned host memory, then the first nzero cleared on the device
 void launch_readback(uint32_t* src, uint32_t* host, int nwords, int nzero, cudaStream_t st);
+// h rows of w words, `pitch` bytes apart, one after the other at dst (device or mapped host memory)
+void launch_pack(uint32_t* dst, const void* src, size_t pitch, int w, int h, cudaStream_t st);
 // fused V(2,2) cycle: per fine level a down kernel (4 passes + restriction) and an
 // up kernel (prolongation + 4 passes; level 0 tail: 1 residual norm + decision,
 // 2 p64 += p, 3 the Krylov dot products, 4 the fused Krylov mode's), and one CTA per
