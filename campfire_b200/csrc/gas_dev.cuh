@@ -282,6 +282,12 @@ __device__ __forceinline__ float div_by_rcp(float x, float d, float r) {
   return __fmaf_rn(e, r, q0);
 }
 
+// x / d from r = RN(1/d) also for tiny x, whose residual div_by_rcp cannot hold exactly: species
+// fade through the whole range of f32, and the advection's limiter compares them
+__device__ __forceinline__ float div_tiny(float x, float d, float r) {
+  return x != 0.f && fabsf(x) < 1e-30f ? x / d : div_by_rcp(x, d, r);
+}
+
 // advect.wgsl:28-34: vel = (s_U, s_V)/dx; RK2 midpoint back-trace (dt < 0 traces forward).
 // The quotient by dx from rdx = RN(1/dx): the IEEE one, except that a velocity of -0 comes
 // out +0, which moves no trace point (g - h * (+-0) = g)

@@ -18,12 +18,6 @@ namespace {
 // RN(1/x) of the divisors every cell shares, once per CTA: their quotients by div_by_rcp, the IEEE ones
 struct Rcp { float cp, sO2, dt, pr, t273; };
 
-// x / d from r = RN(1/d) also for tiny x, whose residual div_by_rcp cannot hold exactly: species
-// fade through the whole range of f32, and the advection's limiter compares them
-__device__ __forceinline__ float div_tiny(float x, float d, float r) {
-  return x != 0.f && fabsf(x) < 1e-30f ? x / d : div_by_rcp(x, d, r);
-}
-
 // what the sources read beside the diffused state; loaded before the diffusion, whose work covers
 // the round trips
 struct CellIn { float2 g; float u0, u1, v0, v1, Tadv; };

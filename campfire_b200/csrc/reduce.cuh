@@ -48,7 +48,7 @@ __device__ __forceinline__ float block_max(float v, float* sh /* >= 32 floats */
 // Publish this CTA's partial; returns true (in every thread) in the CTA that
 // completes the scene's reduction, which then holds the total in *total.
 __device__ __forceinline__ bool scene_reduce(const SceneDesc& S, int tile, int ntiles, double partial,
-                                             double* sh, double* total) {
+                                             double* sh, double* total, int stride = 0) {
   __shared__ int s_last;
   if (threadIdx.x == 0) {
     S.part[tile] = partial;
@@ -58,8 +58,11 @@ __device__ __forceinline__ bool scene_reduce(const SceneDesc& S, int tile, int n
   __syncthreads();
   if (!s_last) return false;
   double v = 0.0;
-  // each thread sums a fixed strided subset in order, then the fixed block tree
-  for (int k = threadIdx.x; k < ntiles; k += blockDim.x) v += __ldcg(S.part + k);
+  // each of the first `stride` threads (0: all) sums a fixed strided subset in order, then the fixed
+  // block tree
+  const int n = stride ? stride : (int)blockDim.x;
+  if ((int)threadIdx.x < n)
+    for (int k = threadIdx.x; k < ntiles; k += n) v += __ldcg(S.part + k);
   const double t = block_sum(v, sh);
   if (threadIdx.x == 0) { *total = t; S.solve->counter = 0u; }
   return true;
