@@ -65,13 +65,13 @@ __device__ __forceinline__ float spline(float l, float l0, float w) {
   return expf(-0.5f * t * t) / (2.5066f * w);
 }
 constexpr int NL = 12;
-constexpr int RENDER_CTAS = 6;   // per SM
+constexpr int RENDER_CTAS = 4;   // per SM: as many as their registers allow, in one wave
 __device__ __forceinline__ float lam(int n) { return 400.0f + ((float)n + 0.5f) * 300.0f / (float)NL; }
 
 // What depends on the wavelength alone, once per CTA (tab[n], fire): the matching functions, the
 // wavelength in metres, Planck's 1.19e-16 / l^5 and the chemiluminescence spectrum. The
 // expressions are the ones a pixel would evaluate, so the values are too.
-struct Wave { V3 cie; float l, c5, chem; };
+struct Wave { V3 cie; float l, rl, c5, chem; };   // rl: RN(1/l)
 // a piece with its rotation, once per CTA
 struct RPiece { float x, y, c, s, half, alive; };
 struct RenderIn {
@@ -81,6 +81,7 @@ struct RenderIn {
   const Wave* tab;
   const RPiece* pcs;
   V3 fire;
+  V3 dark;                 // an unlit gas pixel of this row, encoded
   uint32_t near0, near1;   // pieces that may cover a pixel of this warp (0..31, 32..63)
 };
 
@@ -91,10 +92,20 @@ __device__ V3 gasXYZ(const RenderIn& in, float Tg, float fv, float q) {
   const cfg_params& P = in.S->P;
   V3 xyz = v3(0.f);
   const float c = in.R.chemi * q * P.depth / 12.566f;
+  // soot so thin that its emissivity 1 - exp(-k depth) rounds to zero at the shortest wavelength, and
+  // so at all (expf(-y) is 1 for every f32 y up to 2^-24), times a finite radiance: the air around a fire
+  const float y = 6.3f * fv / in.tab[0].l * P.depth;
+  if (y >= 0.f && y <= 0x1p-25f && fabsf(Tg) < 1e9f) {
+    if (c == 0.f) return xyz;
+    #pragma unroll 4
+    for (int n = 0; n < NL; n++) xyz = xyz + in.tab[n].cie * (c * in.tab[n].chem);
+    return xyz * (300.0f / (float)NL);
+  }
+  fv = fv > 1e30f ? 1e30f : fv;   // opaque already: the quotient by the reciprocal stays finite
   #pragma unroll 4
   for (int n = 0; n < NL; n++) {
     const Wave& w = in.tab[n];
-    const float k = 6.3f * fv / w.l;
+    const float k = div_by_rcp(6.3f * fv, w.l, w.rl);
     float L = (1.0f - expf(-k * P.depth)) * planck(w.l, w.c5, Tg);
     L += c * w.chem;
     xyz = xyz + w.cie * L;
@@ -111,16 +122,11 @@ __device__ V3 greyXYZ(const RenderIn& in, float Ts, float eps) {
   }
   return xyz * (300.0f / (float)NL);
 }
-// :104-109
-__device__ V3 fireLightXYZ(const Wave* tab) {
-  V3 xyz = v3(0.f);
+// :104-109, the term of wavelength n
+__device__ V3 fireLightTerm(const Wave& w, float l) {
   const float l0 = 580.0f * 1e-9f;
   const float b0 = planck(l0, planck_c5(l0), 1400.0f) / 580.0f;
-  for (int n = 0; n < NL; n++) {
-    const float l = lam(n);
-    xyz = xyz + tab[n].cie * planck(tab[n].l, tab[n].c5, 1400.0f) / l / b0;
-  }
-  return xyz * (300.0f / (float)NL);
+  return w.cie * planck(w.l, w.c5, 1400.0f) / l / b0;
 }
 // :110-113
 __device__ __forceinline__ float srgb1(float s) {
@@ -132,11 +138,11 @@ __device__ __forceinline__ V3 srgbEncode(V3 c) {
 }
 // :117-132
 __device__ V3 tonemapXYZ(const RenderIn& in, V3 xyz, V3 base) {
-  const float L = fmax_w(xyz.y * in.R.exposure, 0.f);
-  const float L0 = 0.001f, Lw = 20.0f;
-  const float Ld = logf(1.0f + L / L0) / logf(1.0f + Lw / L0);
   V3 rgb = v3(0.f);
   if (xyz.y > 1e-12f) {
+    const float L = fmax_w(xyz.y * in.R.exposure, 0.f);
+    const float L0 = 0.001f, Lw = 20.0f;
+    const float Ld = logf(1.0f + L / L0) / logf(1.0f + Lw / L0);
     const V3 c = vmax(xyz2rgb(xyz / xyz.y), v3(0.f));
     const float lum = dot3(c, v3(0.2126f, 0.7152f, 0.0722f));
     const V3 pre = c / fmax_w(lum, 1e-6f) * powf(Ld, 2.2f) * 1.6f;
@@ -219,6 +225,8 @@ __device__ float sQ(const SceneDesc& S, float gx, float gy) {
   return mixf(mixf(fQ(S, i, j), fQ(S, i + 1, j), tx), mixf(fQ(S, i, j + 1), fQ(S, i + 1, j + 1), tx), ty);
 }
 
+// the faint sky behind the gas (:236)
+__device__ __forceinline__ V3 skyBase(float uvy) { return mix3(v3(0.006f, 0.006f, 0.010f), v3(0.0015f, 0.0015f, 0.003f), uvy); }
 // :189-273
 __device__ float4 fragment(const RenderIn& in, float wx, float wy, float uvy) {
   const SceneDesc& S = *in.S;
@@ -264,7 +272,8 @@ __device__ float4 fragment(const RenderIn& in, float wx, float wy, float uvy) {
       const float rho = rhoOf(P, Tg);
       const float fv = rho * Yg.w / P.sootDensity;
       xyz = xyz + gasXYZ(in, Tg, fv, sQ(S, gx, gy));
-      rgbAdd = mix3(v3(0.006f, 0.006f, 0.010f), v3(0.0015f, 0.0015f, 0.003f), uvy);
+      rgbAdd = skyBase(uvy);
+      if (!(xyz.y > 1e-12f)) return make_float4(in.dark.x, in.dark.y, in.dark.z, 1.0f);   // tonemapXYZ's unlit case
     }
     const V3 c = tonemapXYZ(in, xyz, rgbAdd);
     return make_float4(c.x, c.y, c.z, 1.0f);
@@ -315,12 +324,14 @@ __device__ float4 fragment(const RenderIn& in, float wx, float wy, float uvy) {
 // spectrum and the pieces' rotations are set up once per CTA instead of per pixel (~200 of the
 // ~230 exponentials of a gas pixel were the matching functions of 12 fixed wavelengths), and each
 // warp first finds which pieces reach its 16x2 pixels. 734x1080 photo of
-// 224x320 with 16 pieces: 252 -> 51 us; 1468x2160 of 352x512 with 40 pieces: 1170 -> 213 us.
+// 224x320 with 16 pieces: 252 -> 45 us (the image kernel alone 50 us
+// at 734x1080 of a burning fire); 1468x2160 of 352x512 with 40 pieces: 1170 -> 170 us. Bound by
+// instruction issue: 12 exponentials and radiances per lit pixel.
 __global__ void __launch_bounds__(256) k_render(const SceneDesc* __restrict__ scenes, int scene, cfg_render_params R,
                                                 const float4* __restrict__ wood, int W, int H, float4* __restrict__ out) {
   __shared__ Wave tab[NL];
   __shared__ RPiece pcs[MAX_PIECES];
-  __shared__ V3 fire;
+  __shared__ V3 fire, term[NL];
   const SceneDesc& S = scenes[scene];
   const int lane = threadIdx.x & 31;
   if (threadIdx.x < NL) {
@@ -328,9 +339,11 @@ __global__ void __launch_bounds__(256) k_render(const SceneDesc* __restrict__ sc
     Wave w;
     w.cie = cie(l);
     w.l = l * 1e-9f;
+    w.rl = __frcp_rn(w.l);
     w.c5 = planck_c5(w.l);
     w.chem = 0.6f * spline(l, 431.0f, 6.0f) + 0.4f * spline(l, 516.0f, 8.0f);
     tab[threadIdx.x] = w;
+    term[threadIdx.x] = fireLightTerm(w, l);
   } else if (threadIdx.x >= 64 && threadIdx.x < 64 + MAX_PIECES) {
     const int n = threadIdx.x - 64;
     RPiece q{0.f, 0.f, 1.f, 0.f, 0.f, 0.f};
@@ -341,20 +354,30 @@ __global__ void __launch_bounds__(256) k_render(const SceneDesc* __restrict__ sc
     pcs[n] = q;
   }
   __syncthreads();
-  if (threadIdx.x == 0) fire = fireLightXYZ(tab);
+  if (threadIdx.x == 0) {
+    V3 xyz = v3(0.f);
+    for (int n = 0; n < NL; n++) xyz = xyz + term[n];
+    fire = xyz * (300.0f / (float)NL);
+  }
   __syncthreads();
-  RenderIn in{scenes + scene, R, wood, tab, pcs, fire, 0u, 0u};
+  RenderIn in{scenes + scene, R, wood, tab, pcs, fire, v3(0.f), 0u, 0u};
   const int tw = (W + 15) / 16, nt = tw * ((H + 15) / 16);
   for (int t = blockIdx.x; t < nt; t += gridDim.x) {
     const int x = (t % tw) * 16 + (threadIdx.x & 15), y = (t / tw) * 16 + (threadIdx.x >> 4);
     const float uvx = ((float)x + 0.5f) / (float)W, uvy = 1.0f - ((float)y + 0.5f) / (float)H;
     const float wx = uvx * R.width / R.zoom + R.camX, wy = uvy * (R.height + R.ground) / R.zoom + R.camY;
-    // the warp's pixels (those past the image too) lie in the box of their corners
-    float x0 = wx, x1 = wx, y0 = wy, y1 = wy;
-    #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      x0 = fminf(x0, __shfl_xor_sync(0xffffffffu, x0, o)); x1 = fmaxf(x1, __shfl_xor_sync(0xffffffffu, x1, o));
-      y0 = fminf(y0, __shfl_xor_sync(0xffffffffu, y0, o)); y1 = fmaxf(y1, __shfl_xor_sync(0xffffffffu, y1, o));
+    // the warp's 16x2 pixels (those past the image too) lie in the box of their corners: each
+    // coordinate is monotonic along its axis
+    const float xa = __shfl_sync(0xffffffffu, wx, 0), xb = __shfl_sync(0xffffffffu, wx, 15);
+    const float ya = __shfl_sync(0xffffffffu, wy, 0), yb = __shfl_sync(0xffffffffu, wy, 16);
+    const float x0 = fminf(xa, xb), x1 = fmaxf(xa, xb), y0 = fminf(ya, yb), y1 = fmaxf(ya, yb);
+    // the row's colour without light (view 0), a component on each of three lanes
+    if (R.view == 0) {
+      const V3 dark = skyBase(uvy);
+      const int l = lane & 15;
+      const float d = srgb1(fmin_w(fmax_w(l == 0 ? dark.x : l == 1 ? dark.y : dark.z, 0.f), 1.f));
+      in.dark = {__shfl_sync(0xffffffffu, d, lane & 16), __shfl_sync(0xffffffffu, d, (lane & 16) + 1),
+                 __shfl_sync(0xffffffffu, d, (lane & 16) + 2)};
     }
     // a square of half side h lies in its centre's box of half side 1.5 h (sqrt 2 and the
     // rounding of the rotation): a piece whose box misses the pixels' covers none of them

@@ -118,3 +118,27 @@ def test_monitor_sums(oracle_mod, nx, ny):
     a, b = g.pressure_residual(), o.pressure_residual()
     assert abs(a - b) <= 1e-9 * max(abs(b), 1e-12)
     g.close()
+
+
+@pytest.mark.parametrize("heat", [0.0, 2e6])
+def test_soot_too_thin_to_shine(heat):
+    # an emissivity 1 - exp(-y) is an exact zero in f32 for y up to 2^-25: at and around the renderer's line for it
+    # the image is the one without soot to the bit, far above the line it is not
+    g = cb.FluidSim(0, {"nx": 48, "ny": 72, "dt": 1e-3}, width=0.8).init()
+    g.writeParams()
+    P = g.params
+    T = np.full(48 * 72, 1200.0, np.float32)
+    SQ = g.readBuffer("SQ").reshape(-1, 2).copy()
+    SQ[:, 1] = heat
+    g.writeBuffer("T", T); g.writeBuffer("SQ", SQ)
+    Y = g.readBuffer("Y").reshape(-1, 4).copy()
+    rho = P["rhoAmb"] * P["Tamb"] / 1200.0
+    images = []
+    for line in (0.0, 1e-20, 0.5, 0.99, 1.01, 1.6, 1e6):
+        # y = 6.3 fv / l * depth at the shortest wavelength, 412.5 nm; fv = rho Y / sootDensity
+        Y[:, 3] = line * 2.0 ** -25 * 412.5e-9 / (6.3 * P["depth"]) * P["sootDensity"] / rho
+        g.writeBuffer("Y", Y)
+        images.append(_image(g, 64, 96, "photo"))
+    g.close()
+    assert all(np.array_equal(a.view(np.uint32), images[0].view(np.uint32)) for a in images[1:-1])
+    assert not np.array_equal(images[-1], images[0])
