@@ -176,7 +176,6 @@ int Engine::init(int device, int n, const int* nx, const int* ny, const double* 
   CFG_CUDA(prepare_mg_coarse(coarse_smem_));
   CFG_CUDA(prepare_coarse_factor(cf_smem_));
   CFG_CUDA(prepare_diffuse_sources());
-  CFG_CUDA(prepare_radiation());
   CFG_CUDA(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
   CFG_CUDA(cudaStreamCreateWithFlags(&body_stream_, cudaStreamNonBlocking));
   CFG_CUDA(cudaStreamCreateWithFlags(&side_stream_, cudaStreamNonBlocking));

@@ -5,6 +5,8 @@
 #include "kernels.h"
 #include "reduce.cuh"
 
+#include <cooperative_groups.h>
+
 namespace cfg {
 
 // u -= dt (1/rho_f) grad p; ghost -p at the open sides/top, closed faces 0.
@@ -276,24 +278,25 @@ __global__ void __launch_bounds__(256) k_emission(const SceneDesc* __restrict__ 
       make_float2(kap * P.sigma * (T2v * T2v - T4a) / 3.14159265f, 6.3f * fv / 580e-9f * planck580(Tg));
 }
 
-// :64-158 one CTA per wood face or floor probe. Rays in tiles of up to RAD_RT; a tile's rays go
-// through the same phases together, once for the way from their origin and once after the
-// floor's bounce: (1) the first piece hit, G lanes per ray sharing the pieces; (2) the samples
-// along the rays, RAD_CH per ray at a time, by all warps but the last RAD_RT threads', which at the
-// same time (3) add the chunk before to their ray's sums in the order of the reference's loop.
-// Bound by the latency of one target's phases (about one CTA per SM for 16 pieces): one thread
-// per ray marching its samples alone was two warps per SM in a serial chain of 200-600 samples.
-// With
-// 64 rays and 16 pieces: 453 -> 35 us at 224x320, 719 -> 46 us at 352x512, k_emission included;
-// 40 pieces at 352x512: 721 -> 55 us.
+// :64-158 a cluster of CTAs per wood face or floor probe, RAD_RT rays at a time each (1024 rays are the
+// most; up to RAD_CL CTAs share them). The rays of a CTA go through the same phases
+// together, once for the way from their origin and once after the floor's bounce: (1) the first
+// piece hit, G lanes per ray sharing the pieces; (2) the samples along the rays, RAD_CH per ray at
+// a time, by all warps but the last, which at the same time (3) adds the chunk before to its rays'
+// sums in the order of the reference's loop. The first CTA adds the rays' shares in the
+// reference's tree. Bound by instruction issue and by the spread of the rays' lengths over the
+// SMs: one thread per ray marching its samples alone was two warps per SM in a serial chain of
+// 200-600 samples, one CTA of 1024 threads per target left the longest targets' SMs last.
+// With 64 rays and 16 pieces: 453 -> 29 us at 224x320 (35 with a CTA per target); 40 pieces at
+// 352x512: 721 -> 50 us (55); k_emission's 7 us included.
 namespace {
-constexpr int RAD_RT = 64, RAD_CH = 64, RAD_THREADS = 1024;
+constexpr int RAD_CH = 64, RAD_THREADS = 256, RAD_CL = 8;
 constexpr int RAD_ROW = RAD_CH + 1;   // terms of a ray in shared memory: odd, so that a warp of rays reads 32 banks
-constexpr size_t RAD_SMEM = (size_t)2 * RAD_RT * RAD_ROW * sizeof(float2);
 struct Ray { float ox, oy, dx, dy, tOut, tFloor, rns, hitT; int ns, next; };   // next: 0 done, 1 bounces
 }
+template <int RAD_RT>
 __global__ void __launch_bounds__(RAD_THREADS) k_radiation(const SceneDesc* __restrict__ scenes, int scene, int NRAY) {
-  extern __shared__ __align__(16) float2 terms[];   // [2][RAD_RT][RAD_ROW]
+  __shared__ __align__(16) float2 terms[2 * RAD_RT * RAD_ROW];
   __shared__ Piece sp[MAX_PIECES];
   __shared__ float sc[MAX_PIECES], ss[MAX_PIECES];
   __shared__ float sq[1024], sv[1024];
@@ -308,18 +311,21 @@ __global__ void __launch_bounds__(RAD_THREADS) k_radiation(const SceneDesc* __re
   if ((int)threadIdx.x < np) { sc[threadIdx.x] = cosf(sp[threadIdx.x].angle); ss[threadIdx.x] = sinf(sp[threadIdx.x].angle); }
   __syncthreads();
   const float PI = 3.14159265f;
-  const uint32_t tgt = blockIdx.x;
+  cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+  const int ncta = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+  const uint32_t tgt = blockIdx.x / ncta;
   const uint32_t nFaces = (uint32_t)np * 4u;
   const int nx = S.nx, ny = S.ny, pcw = S.pc;
   const float dx = P.dx, rdx = __frcp_rn(dx);
   const float2* E = reinterpret_cast<const float2*>(S.Yw);
   const bool face = tgt < nFaces;
   const bool valid = face ? sp[tgt / 4u].alive > 0.f : tgt - nFaces < (uint32_t)N_FLOOR;
-  if (!valid) return;   // the same in every thread: nothing of this target is written
+  if (!valid) return;   // the same in every thread of the cluster: nothing of this target is written
+  cl.sync();            // every CTA runs: the first one's shared memory may be written
   const int RT = min(NRAY, RAD_RT);
   const int G = min(RAD_THREADS / RT, 32);   // lanes per ray in phase 1 (both powers of two)
-  const int tid = threadIdx.x, sum0 = RAD_THREADS - RAD_RT;   // threads from sum0 on add
-  for (int r0 = 0; r0 < NRAY; r0 += RT) {
+  const int tid = threadIdx.x, sum0 = RAD_THREADS - 32;   // the last warp adds
+  for (int r0 = rank * RT; r0 < NRAY; r0 += ncta * RT) {
     float J = 0.f, Jv = 0.f, Twall = P.Tamb, cosn = 0.f;   // of ray r0 + tid - sum0 in the adding threads
     const int mine = tid - sum0;
     if (mine >= 0 && mine < RT) {
@@ -412,7 +418,8 @@ __global__ void __launch_bounds__(RAD_THREADS) k_radiation(const SceneDesc* __re
               const int gi = wgsl_i32(div_by_rcp(px, dx, rdx)), gj = wgsl_i32(div_by_rcp(py, dx, rdx));
               float2 g = make_float2(0.f, 0.f);
               if (!(gi < 0 || gj < 0 || gi >= nx || gj >= ny)) g = E[gj * pcw + gi];
-              buf[r * RAD_ROW + e % RAD_CH] = make_float2(g.x * q.tOut / fns, g.y * q.tOut / fns);
+              // emission fades to nothing in clear air: its quotients stay exact
+              buf[r * RAD_ROW + e % RAD_CH] = make_float2(div_tiny(g.x * q.tOut, fns, q.rns), div_tiny(g.y * q.tOut, fns, q.rns));
             }
           }
         } else if (k > 0 && mine < RT) {
@@ -436,14 +443,15 @@ __global__ void __launch_bounds__(RAD_THREADS) k_radiation(const SceneDesc* __re
       Twall = ray[mine].hitT;
       const float wgt = PI / (float)NRAY * cosn;
       const float T2v = Twall * Twall;
-      sq[r0 + mine] = wgt * (0.5f * P.sigma * T2v * T2v + 2.f * J);
-      sv[r0 + mine] = wgt * (2.f * Jv);
+      cl.map_shared_rank(sq, 0)[r0 + mine] = wgt * (0.5f * P.sigma * T2v * T2v + 2.f * J);
+      cl.map_shared_rank(sv, 0)[r0 + mine] = wgt * (2.f * Jv);
     }
   }
-  __syncthreads();
+  cl.sync();
+  if (rank != 0) return;
   const int li = tid;
   for (int s = NRAY / 2; s > 0; s >>= 1) {
-    if (li < s) { sq[li] += sq[li + s]; sv[li] += sv[li + s]; }
+    for (int k = li; k < s; k += RAD_THREADS) { sq[k] += sq[k + s]; sv[k] += sv[k + s]; }
     __syncthreads();
   }
   if (li == 0) {
@@ -546,13 +554,25 @@ void launch_cfl_update(SceneDesc* scenes, int nscenes, const double* dxd, const 
 void launch_geometry(const SceneDesc* scenes, const Work* work, int ntiles, cudaStream_t st) {
   if (ntiles > 0) k_geometry<<<ntiles, GEO_TX * GEO_TY, 0, st>>>(scenes, work);
 }
-cudaError_t prepare_radiation() {
-  return cudaFuncSetAttribute(k_radiation, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RAD_SMEM);
-}
 void launch_radiation(const SceneDesc* scenes, int scene, int nx, int ny, int ntargets, int nray, cudaStream_t st) {
   if (ntargets <= 0) return;
   k_emission<<<dim3((nx + 31) / 32, (ny + 7) / 8), 256, 0, st>>>(scenes, scene);
-  k_radiation<<<ntargets, RAD_THREADS, RAD_SMEM, st>>>(scenes, scene, nray);
+  // 16 rays per CTA spread few targets over the chip; from four such CTAs per SM on, 32 rays keep the
+  // adding warp full. Both, whole pass: 160x224 with 16 pieces 25 and 31 us, 224x320 with 16 29 and
+  // 37 us, 352x512 with 40 58 and 50 us.
+  const int rt = (long)ntargets * nray > 4L * 148 * 16 ? 32 : 16;
+  const int ncta = nray / rt < 1 ? 1 : nray / rt > RAD_CL ? RAD_CL : nray / rt;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ntargets * ncta);
+  cfg.blockDim = dim3(RAD_THREADS);
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = ncta; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  if (rt == 32) cudaLaunchKernelEx(&cfg, k_radiation<32>, scenes, scene, nray);
+  else cudaLaunchKernelEx(&cfg, k_radiation<16>, scenes, scene, nray);
 }
 void launch_budgets(const SceneDesc* scenes, int scene, int cells, double* out, cudaStream_t st) {
   k_budgets<<<monitor_ctas(cells), 256, 0, st>>>(scenes, scene, out);

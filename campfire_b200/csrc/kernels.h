@@ -161,7 +161,6 @@ void launch_project(SceneDesc* scenes, const Work* work, int ntiles, bool fp64, 
 void launch_cfl_update(SceneDesc* scenes, int nscenes, const double* dxd, const double* alpha, cudaStream_t st);
 void launch_geometry(const SceneDesc* scenes, const Work* work, int ntiles, cudaStream_t st);
 void launch_radiation(const SceneDesc* scenes, int scene, int nx, int ny, int ntargets, int nray, cudaStream_t st);
-cudaError_t prepare_radiation();   // its dynamic shared memory, once per device before the first launch
 // FP64 budgets of one scene into out[8] (device)
 void launch_budgets(const SceneDesc* scenes, int scene, int cells, double* out, cudaStream_t st);
 // ||r||2 and ||rhs||2 of level 0 of one scene into out[2] (device, FP64)

@@ -120,6 +120,12 @@ def test_monitor_sums(oracle_mod, nx, ny):
     g.close()
 
 
+@pytest.mark.parametrize("npieces,nray", [(0, 256), (1, 128), (5, 64), (3, 8)])
+def test_radiation_rays_shared_by_a_cluster(oracle_mod, npieces, nray):
+    # few targets: 16 rays per CTA, one to eight CTAs a target, one or two rounds each
+    test_radiation_over_rays_and_pieces(oracle_mod, 48, 72, npieces, nray)
+
+
 @pytest.mark.parametrize("heat", [0.0, 2e6])
 def test_soot_too_thin_to_shine(heat):
     # an emissivity 1 - exp(-y) is an exact zero in f32 for y up to 2^-25: at and around the renderer's line for it
