@@ -91,8 +91,8 @@ __device__ __forceinline__ bool scene_idle(const SolveState* ss) { return *(cons
 
 // Tile staging on two barriers around the wait on the previous kernel. stage_coef
 // (before the wait in a one-scene engine, which also waits for them and builds the stencils
-// before the wait, with the state copies' tensor maps prefetched; else once the scene's flag
-// says it still cycles): one thread initialises both barriers and requests the coefficients
+// before the wait, with the state copies' tensor maps prefetched; else after it, with
+// stage_state, once the scene's flag says it still cycles): one thread initialises both barriers and requests the coefficients
 // ax, ay on bar[0]; they are built before the pressure loop and written by no loop kernel
 // (the loop is entered through a full dependency: a graph node or a memset). stage_state
 // (after the wait): p from map `pkind`, rhs and the coarse p under the tile on bar[1]; with
@@ -110,9 +110,11 @@ __device__ __forceinline__ void stage_coef(const SceneDesc& S, int level, const 
     tma_load_2d(t.ay, tmap_of(S, level, TM_AY), t.sx, t.sy, &bar[0]);
   }
 }
-// the tensor maps of stage_state's copies into the descriptor cache (before the wait)
-__device__ __forceinline__ void prefetch_state_maps(const SceneDesc& S, int level, int pkind, bool coarse) {
+// the tensor maps of stage_state's copies (coef: and of stage_coef's) into the descriptor cache
+// (before the wait)
+__device__ __forceinline__ void prefetch_state_maps(const SceneDesc& S, int level, int pkind, bool coarse, bool coef = false) {
   if (threadIdx.x == 0) {
+    if (coef) { tmap_prefetch(tmap_of(S, level, TM_AX)); tmap_prefetch(tmap_of(S, level, TM_AY)); }
     tmap_prefetch(tmap_of(S, level, pkind));
     tmap_prefetch(tmap_of(S, level, TM_RHS));
     if (coarse) tmap_prefetch(tmap_of(S, level + 1, TM_PC));
@@ -475,8 +477,25 @@ __global__ void __launch_bounds__(256, MINB) k_mg_down(const SceneDesc* __restri
   }
   // below level 0 the level's p is zero on entry (the restriction above zeroes it)
   const bool pz = level > 0;
+  // several scenes: mostly more tiles than fit at once, so nothing is gained before the wait; what the
+  // copies depend on is read in one round, and all of them are requested together, their tensor maps
+  // prefetched (64 uneven scenes: 3878 -> 3826 us per step)
+  PcgPrev pv{};
+  bool live = true;
+  if (!spec) {
+    prefetch_state_maps(S, level, TM_P, false, true);
+    pdl_wait();
+    if (on) {
+      live = *(volatile int*)&ss->active != 0;
+      if (PCG) pv = pcg_load(ss);
+    }
+  }
   f2 p[2];
   zero_sp(sp, p);
+  if (!spec && on && live && threadIdx.x == 0) {
+    stage_coef(S, level, t, bar);
+    stage_state(S, level, TM_P, t, !(PCG && pv.cycles >= 1), nullptr, 0, 0, bar, !pz);
+  }
   __syncthreads();
   const bool idle = on && spec && s_idle;
   // one scene: the stencils, which depend on the coefficients alone, are built before the wait
@@ -484,24 +503,27 @@ __global__ void __launch_bounds__(256, MINB) k_mg_down(const SceneDesc* __restri
   c.nz = nz;
   bool ok = true;
   if (on && spec && !idle && (ok = tile_wait(&bar[0], ctl))) item_stencils(t, L, q, c);
-  pdl_wait();
+  if (spec) pdl_wait();
   if (count_iter && blockIdx.x == 0 && threadIdx.x == 0) loop_count(ctl);
   if (!on || !ok || idle) return;
-  if (!spec) {
-    if (*(volatile int*)&ss->active == 0) return;
-    stage_coef(S, level, t, bar);
-    __syncthreads();
+  if (spec) {
+    if (PCG) pv = pcg_load(ss);
+    live = *(volatile int*)&ss->active != 0;
+  } else if (!live) {
+    return;
   }
-  PcgPrev pv{};
-  if (PCG) pv = pcg_load(ss);
-  const bool live = *(volatile int*)&ss->active != 0;
   const bool upd = PCG && pv.cycles >= 1;   // an update of the previous cycle is pending
-  stage_state(S, level, TM_P, t, !upd, nullptr, 0, 0, bar, !pz);
+  if (spec) stage_state(S, level, TM_P, t, !upd, nullptr, 0, 0, bar, !pz);
   float4 rv = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (PCG && upd && live) rv = pcg_rhs(S, L, q, pv);
+  const bool mine = in_tile(q, x0, y0);
+  if (PCG && upd && live) {
+    rv = pcg_rhs(S, L, q, pv);
+    // the pending direction and pressure (read and written by this item alone): with several scenes beside
+    // the copies, with one after the results that the next kernel waits for
+    if (!spec && mine) pcg_dir(S, L, q, pv);
+  }
   if (!(spec ? tile_wait(&bar[1], ctl) : tile_wait2(bar, ctl, [&] { item_stencils(t, L, q, c); })) || !live)
     return;
-  const bool mine = in_tile(q, x0, y0);
   f2 rhs[2];
   if (upd) {
     // rhs0 of the tile also to global, for the up kernel's staging
@@ -554,8 +576,7 @@ __global__ void __launch_bounds__(256, MINB) k_mg_down(const SceneDesc* __restri
       }
     }
   }
-  // the pending direction and pressure (read and written by this item alone)
-  if (PCG && upd && mine) pcg_dir(S, L, q, pv);
+  if (PCG && spec && upd && mine) pcg_dir(S, L, q, pv);
 }
 
 // ------------------------------------------------------------------ up: prolong + 4 passes (+ level-0 tail)
@@ -590,6 +611,20 @@ __global__ void __launch_bounds__(256, MINB) k_mg_up(const SceneDesc* __restrict
   const bool on = S.enabled;   // host-written, constant during the step
   SolveState* ss = S.solve;
   constexpr bool spec = ONE;   // as in k_mg_down
+  PcgPrev pv{};
+  bool live = true;
+  if (!spec) {
+    prefetch_state_maps(S, level, TM_PB, true, true);
+    pdl_wait();
+    if (on) {
+      live = *(volatile int*)&ss->active != 0;
+      if (KRY) pv = pcg_load(ss);
+      if (live && threadIdx.x == 0) {
+        stage_coef(S, level, t, bar);
+        stage_state(S, level, TM_PB, t, true, scp, cx, cy, bar);
+      }
+    }
+  }
   __shared__ int s_idle;
   if (on && spec && threadIdx.x == 0) {
     const bool z = scene_idle(ss);
@@ -613,20 +648,18 @@ __global__ void __launch_bounds__(256, MINB) k_mg_up(const SceneDesc* __restrict
     pl = ring_plan(t, L, C, cx, cy);
   };
   if (on && spec && !idle && (ok = tile_wait(&bar[0], ctl))) prepare();
-  pdl_wait();
+  if (spec) pdl_wait();
   if (!on || !ok || idle) return;
-  if (!spec) {
-    if (*(volatile int*)&ss->active == 0) return;
-    stage_coef(S, level, t, bar);
-    __syncthreads();
+  if (spec) {
+    stage_state(S, level, TM_PB, t, true, scp, cx, cy, bar);
+    live = *(volatile int*)&ss->active != 0;
+  } else if (!live) {
+    return;
   }
-  stage_state(S, level, TM_PB, t, true, scp, cx, cy, bar);
-  const bool live = *(volatile int*)&ss->active != 0;
   // fused Krylov mode: the solve state and this thread's stored r, q, Lz, read beside the copies
-  PcgPrev pv{};
   double r0[2] = {0.0, 0.0}, q0[2] = {0.0, 0.0}, lz0[2] = {0.0, 0.0};
   if (KRY) {
-    pv = pcg_load(ss);
+    if (spec) pv = pcg_load(ss);
     #pragma unroll
     for (int m = 0; m < 2; m++) {
       const int e = threadIdx.x + 256 * m;
