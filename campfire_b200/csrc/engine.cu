@@ -163,7 +163,7 @@ int Engine::init(int device, int n, const int* nx, const int* ny, const double* 
     sc.lc = choose_lc(sc, coarse_cells_, 0, block_cap_, true);
     coarse_smem_ = std::max(coarse_smem_, coarse_smem_bytes(sc.lnx, sc.lny, sc.lc, sc.nlev));
     const int cn = sc.lnx[L - 1] * sc.lny[L - 1], cbw = sc.lnx[L - 1];
-    if (cbw <= 32) { cf_smem_ = std::max(cf_smem_, coarse_factor_smem(cn, cbw)); cf_bw_ = std::max(cf_bw_, cbw); }
+    if (cbw <= 32) { cf_smem_ = std::max(cf_smem_, coarse_factor_smem(cn)); cf_bw_ = std::max(cf_bw_, cbw); }
   }
   int ndev = 0;
   const cudaError_t e = cudaGetDeviceCount(&ndev);

@@ -1350,22 +1350,22 @@ constexpr size_t CF_SMEM_BUDGET = 200 * 1024;
 
 // Columns of the inverse solved per pass: all n when the working columns fit the
 // shared-memory budget beside the band, else 128 per pass.
+constexpr int CF_ROW = 2 * CF_MAXBW + 5;   // floats per row beside its columns: the widest band, the column, 1 / L_ii
 __host__ __device__ inline int coarse_factor_cols(int n) {
-  const size_t W = CF_MAXBW + 1;   // the widest band
-  return ((size_t)n * n + (size_t)n * W + n) * sizeof(float) <= CF_SMEM_BUDGET ? n : 128;
+  return (size_t)n * (n + CF_ROW) * sizeof(float) <= CF_SMEM_BUDGET ? n : 128;
 }
-size_t coarse_factor_smem(int n, int bw) {
-  const int C = coarse_factor_cols(n);
-  return ((size_t)n * (bw + 1) + n + (size_t)n * C) * sizeof(float);
-}
+size_t coarse_factor_smem(int n) { return (size_t)n * (coarse_factor_cols(n) + CF_ROW) * sizeof(float); }
 
-// The inverse of the coarsest operator of each scene: the banded matrix is
-// factored L L^T by one warp (right-looking; lane l owns row jc + 1 + l of the
-// trailing band, takes the new column's l_kj from the lanes that computed them
-// by shuffle and updates its row from registers), then each thread solves
-// L L^T x = e_c for its column c with the band's sliding window in registers
-// (BWM = the band width bound, a compile-time size so the window stays in
-// registers); the forward result is kept in shared memory (Y[i * C + t]).
+// The inverse of the coarsest operator of each scene: the banded matrix is factored L L^T by one
+// warp whose lanes hold the rows of the trailing band in registers (a row enters BWM columns before
+// its own; the new column's l_kj by shuffle), then each thread solves L L^T x = e_c for its column
+// c: forward with the next BWM rows' sums in registers, each y_i subtracted from all of them at
+// once, backward with the last BWM x in registers; the forward result is kept in shared memory
+// (Y[i * C + t]). Padded with zeros to BWM, rows of the band and columns of L are plain 16-byte
+// loads; a zero coefficient changes no sum. Bound by latency: a warp's chain of square root, quotient
+// and shuffle per column, then of one fused multiply-add per band entry and row. With the band
+// packed and every load behind its own bounds test an inverse of 8x12 took 58 us, of 12x17 216, of
+// 16x16 500; now 33, 111 and 113.
 // pipelined = 0: the inverse of this step's operator into the half the cycles use (direct_ok);
 // pipelined = 1: into the other half for the next step (direct_ok_next), while this step's
 // cycles use the current half.
@@ -1377,7 +1377,8 @@ __global__ void __launch_bounds__(CF_THREADS) k_coarse_factor(const SceneDesc* _
   const SceneDesc& S = scenes[blockIdx.x];
   if (!S.enabled) return;
   const LevelDesc L = S.lev[S.nlev - 1];
-  const int n = L.nx * L.ny, bw = L.nx, W = bw + 1;
+  constexpr int WS = BWM + 4;
+  const int n = L.nx * L.ny, bw = L.nx;
   int* ok_flag = pipelined ? &S.solve->direct_ok_next : &S.solve->direct_ok;
   const int ld = cinv_ld(n);
   float* cinv = S.cinv + (size_t)(pipelined ? 1 - S.solve->cinv_cur : S.solve->cinv_cur) * n * ld;
@@ -1385,14 +1386,16 @@ __global__ void __launch_bounds__(CF_THREADS) k_coarse_factor(const SceneDesc* _
     if (threadIdx.x == 0) *ok_flag = 0;
     return;
   }
-  float* band = cf_smem;                 // n * W
-  float* rinv = band + (size_t)n * W;    // n
+  // L below A in place: band[i * WS + m] = A[i][i - BWM + m], the diagonal at m = BWM, zeros left of the band
+  float* band = cf_smem;                 // n * WS
+  float* col = band + n * WS;            // n * BWM: col[i * BWM + m] = L[i + 1 + m][i]
+  float* rinv = col + n * BWM;           // n
   float* Y = rinv + n;                   // n * C
   const int C = coarse_factor_cols(n);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int e = tid; e < n * W; e += CF_THREADS) band[e] = 0.f;
+  for (int e = tid; e < n * WS; e += CF_THREADS) band[e] = 0.f;
   __syncthreads();
-  // lower band: band[k*W + d] = A[k][k-d]; the diagonal is kept in rinv[] until dmax is known
+  // the diagonal is kept in rinv[] until dmax is known
   for (int k = tid; k < n; k += CF_THREADS) {
     const int i = k % L.nx, j = k / L.nx;
     const float w = L.ax[j * L.pu + i], e = L.ax[j * L.pu + i + 1];
@@ -1404,48 +1407,62 @@ __global__ void __launch_bounds__(CF_THREADS) k_coarse_factor(const SceneDesc* _
     if (j < L.ny - 1) diag += no; else diag += 2.f * no;
     rinv[k] = diag;
     if (diag > 0.f) {
-      band[k * W] = diag;
-      if (i > 0) band[k * W + 1] = -w;
-      if (j > 0) band[k * W + bw] = -so;
+      float* r = band + k * WS + BWM;
+      r[0] = diag;
+      if (i > 0) r[-1] = -w;
+      if (j > 0) r[-bw] = -so;
     }
   }
   __syncthreads();
-  if (tid == 0) {
+  if (warp == 0) {
     float m = 0.f;
-    for (int k = 0; k < n; k++) m = fmaxf(m, rinv[k]);
-    s_dmax = m;
-    s_ok = m > 0.f ? 1 : 0;
+    for (int k = lane; k < n; k += 32) m = fmaxf(m, rinv[k]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if (lane == 0) { s_dmax = m; s_ok = m > 0.f ? 1 : 0; }
   }
   __syncthreads();
   const float dmax = s_dmax, thr = 1e-6f * dmax;
   for (int k = tid; k < n; k += CF_THREADS)
-    if (!(rinv[k] > 0.f)) band[k * W] = dmax;
+    if (!(rinv[k] > 0.f)) band[k * WS + BWM] = dmax;
   __syncthreads();
   if (warp == 0 && s_ok) {
+    // row i lives in lane i % 32 from column i - BWM on: a[m] = A[i][jc + m]; in: the row that enters next
+    float a[WS], in[WS];
+    auto row = [&](int i, float (&v)[WS]) {
+      const float4* r = reinterpret_cast<const float4*>(band + min(i, n - 1) * WS);
+#pragma unroll
+      for (int m = 0; m < WS / 4; m++) { const float4 q = r[m]; v[4 * m] = q.x; v[4 * m + 1] = q.y; v[4 * m + 2] = q.z; v[4 * m + 3] = q.w; }
+    };
+    row(lane, in);
+#pragma unroll
+    for (int m = 0; m <= BWM; m++) a[m] = in[m];
+    // row r < BWM starts at column 0: its first BWM - r entries lie left of the matrix
+    for (int r = lane; r < BWM; r++) {
+#pragma unroll
+      for (int m = 0; m < BWM; m++) a[m] = a[m + 1];
+    }
+    row(BWM, in);
     for (int jc = 0; jc < n; jc++) {
-      const float piv = band[jc * W];
-      if (!(piv > thr)) {   // every lane read the same pivot
+      const float piv = __shfl_sync(0xffffffffu, a[0], jc & 31);
+      if (!(piv > thr)) {   // every lane has the same pivot
         if (lane == 0) s_ok = 0;
         break;
       }
+      const bool enters = lane == ((jc + BWM) & 31);
+#pragma unroll
+      for (int m = 0; m <= BWM; m++) a[m] = enters ? in[m] : a[m];
+      row(jc + 1 + BWM, in);
       const float ljj = sqrtf(piv);
-      const int i = jc + 1 + lane;
-      const bool mine = lane < bw && i < n;
-      float lij = 0.f;
-      if (mine) lij = band[i * W + (i - jc)] / ljj;
-      // A[i][k] -= l_ij l_kj for k = jc + 1 + m <= i: l_kj from lane m, A[i][k] at band[i*W + lane - m]
-      float lk[BWM], tg[BWM];
+      const int d = 1 + ((lane - jc - 1) & 31), i = jc + d;
+      const bool mine = d <= bw && i < n;
+      const float q = a[0] / ljj, lij = mine ? q : 0.f;
+      if (lane == 0) band[jc * WS + BWM] = ljj;
+      if (mine) band[i * WS + BWM - d] = lij;
+      // A[i][k] -= l_ij l_kj for k = jc + 1 + m <= i (the entries past i are never read), l_kj from row k's
+      // lane; zeros in the lanes of no such row
 #pragma unroll
-      for (int m = 0; m < BWM; m++) lk[m] = __shfl_sync(0xffffffffu, lij, m);
-#pragma unroll
-      for (int m = 0; m < BWM; m++) tg[m] = (mine && m <= lane) ? band[i * W + (lane - m)] : 0.f;
-      __syncwarp();
-      if (lane == 0) band[jc * W] = ljj;
-      if (mine) band[i * W + (i - jc)] = lij;
-#pragma unroll
-      for (int m = 0; m < BWM; m++)
-        if (mine && m <= lane) band[i * W + (lane - m)] = __fmaf_rn(-lij, lk[m], tg[m]);
-      __syncwarp();
+      for (int m = 0; m < BWM; m++) a[m] = __fmaf_rn(-lij, __shfl_sync(0xffffffffu, lij, (jc + 1 + m) & 31), a[m + 1]);
     }
   }
   __syncthreads();
@@ -1453,43 +1470,49 @@ __global__ void __launch_bounds__(CF_THREADS) k_coarse_factor(const SceneDesc* _
     if (tid == 0) *ok_flag = 0;
     return;
   }
-  for (int k = tid; k < n; k += CF_THREADS) rinv[k] = 1.0f / band[k * W];
+  for (int k = tid; k < n; k += CF_THREADS) rinv[k] = 1.0f / band[k * WS + BWM];
+  for (int e = tid; e < n * BWM; e += CF_THREADS) {
+    const int i = e / BWM, m = e % BWM;
+    col[e] = i + 1 + m < n ? band[(i + 1 + m) * WS + BWM - 1 - m] : 0.f;
+  }
   __syncthreads();
   for (int c0 = 0; c0 < n; c0 += C) {
-    const int t = tid, c = c0 + tid;
-    if (t < C && c < n) {
-      float* y = Y + t;   // y[i * C]
-      for (int i = 0; i < c; i++) y[i * C] = 0.f;
-      // forward: y_i = (e_c[i] - sum_{k = max(c, i-bw)}^{i-1} L[i][k] y_k) / L[i][i], k ascending;
-      // win[m] = y_{i-1-m}
-      float win[BWM];
+    const int c = c0 + tid;
+    if (tid < C && c < n) {
+      float* y = Y + tid;   // y[i * C]
+      // rows above the warp's first column hold zeros
+      const int first = c0 + (tid & ~31);
+      float l[BWM], v[BWM + 1];
+      auto column = [&](int i) {
+        const float4* r = reinterpret_cast<const float4*>(col + i * BWM);
 #pragma unroll
-      for (int m = 0; m < BWM; m++) win[m] = 0.f;
-      for (int i = c; i < n; i++) {
-        float sum = i == c ? 1.f : 0.f;
+        for (int m = 0; m < BWM / 4; m++) { const float4 q = r[m]; l[4 * m] = q.x; l[4 * m + 1] = q.y; l[4 * m + 2] = q.z; l[4 * m + 3] = q.w; }
+      };
+      // forward: y_i = v_i / L[i][i], then v_k -= L[k][i] y_i for k = i+1 .. i+bw; v[m] is row i+m's sum
 #pragma unroll
-        for (int m = BWM - 1; m >= 0; m--)
-          if (m < bw && i - 1 - m >= c) sum = __fmaf_rn(-band[i * W + (m + 1)], win[m], sum);
-        const float yi = sum * rinv[i];
+      for (int m = 0; m <= BWM; m++) v[m] = first + m == c ? 1.f : 0.f;
+      for (int i = first; i < n; i++) {
+        column(i);
+        const float yi = v[0] * rinv[i];
         y[i * C] = yi;
 #pragma unroll
-        for (int m = BWM - 1; m > 0; m--) win[m] = win[m - 1];
-        win[0] = yi;
+        for (int m = 0; m < BWM; m++) v[m] = __fmaf_rn(-l[m], yi, v[m + 1]);
+        v[BWM] = i + 1 + BWM == c ? 1.f : 0.f;
       }
       // backward: x_i = (y_i - sum_{k = i+1}^{min(n-1, i+bw)} L[k][i] x_k) / L[i][i], k ascending;
-      // win[m] = x_{i+1+m}
+      // v[m] = x_{i+1+m}
 #pragma unroll
-      for (int m = 0; m < BWM; m++) win[m] = 0.f;
+      for (int m = 0; m < BWM; m++) v[m] = 0.f;
       for (int i = n - 1; i >= 0; i--) {
-        float sum = y[i * C];
+        column(i);
+        float x = i >= first ? y[i * C] : 0.f;
 #pragma unroll
-        for (int m = 0; m < BWM; m++)
-          if (m < bw && i + 1 + m <= n - 1) sum = __fmaf_rn(-band[(i + 1 + m) * W + (m + 1)], win[m], sum);
-        const float xi = sum * rinv[i];
-        cinv[(size_t)i * ld + c] = xi;
+        for (int m = 0; m < BWM; m++) x = __fmaf_rn(-l[m], v[m], x);
+        x *= rinv[i];
+        cinv[(size_t)i * ld + c] = x;
 #pragma unroll
-        for (int m = BWM - 1; m > 0; m--) win[m] = win[m - 1];
-        win[0] = xi;
+        for (int m = BWM - 1; m > 0; m--) v[m] = v[m - 1];
+        v[0] = x;
       }
     }
     __syncthreads();

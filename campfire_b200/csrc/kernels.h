@@ -143,8 +143,8 @@ void launch_cinv_swap(const SceneDesc* scenes, int nscenes, cudaStream_t st);
 // (mod 32), so that the four rows a warp reads at once in the coarse block's product fall in
 // different shared-memory banks (ld * 4 bytes stays a multiple of 16 for the bulk copies)
 __host__ __device__ constexpr int cinv_ld(int n) { return n <= 8 ? 8 : (n - 8 + 31) / 32 * 32 + 8; }
-// dynamic shared memory of k_coarse_factor for a coarsest level of n cells and band width bw
-size_t coarse_factor_smem(int n, int bw);
+// dynamic shared memory of k_coarse_factor for a coarsest level of n cells
+size_t coarse_factor_smem(int n);
 cudaError_t prepare_coarse_factor(size_t smem);
 // ||rhs||^2 (FP64 mode: ||rhs64||^2) of level 0; arms the pressure loop
 void launch_bnorm(const SceneDesc* scenes, const Work* work, int ntiles, SolveCtl* ctl, bool fp64, cudaStream_t st);
