@@ -15,8 +15,9 @@ namespace cfg {
 
 namespace {
 
-// RN(1/x) of the divisors every cell shares, once per CTA: their quotients by div_by_rcp, the IEEE ones
-struct Rcp { float cp, sO2, dt, pr, t273; };
+// what every cell shares, once per CTA: RN(1/x) of the divisors (their quotients by div_by_rcp, the
+// IEEE ones) and powf(Tamb, 4)
+struct Rcp { float cp, sO2, dt, pr, t273, Tamb4; };
 
 // what the sources read beside the diffused state; loaded before the diffusion, whose work covers
 // the round trips
@@ -31,9 +32,8 @@ __device__ __forceinline__ float rhoD(const cfg_params& P, const Rcp& R, float T
 // sources.wgsl:34-157 for one gas cell; returns false for a cell inside wood
 struct SrcOut { float T; float4 Y; float S, qrel, qrad, tpeak; bool solid; };
 
-// Tamb4 = powf(P.Tamb, 4) (the radiation's ambient term, the same for every cell of the scene)
 __device__ __forceinline__ SrcOut sources_cell(const SceneDesc& S, const cfg_params& P, const Rcp& R, const CellIn& in, int i, int j,
-                                               float Tc, float4 Yc, float Tamb4) {
+                                               float Tc, float4 Yc) {
   SrcOut o; o.qrel = 0.f; o.qrad = 0.f; o.tpeak = 0.f; o.solid = false; o.S = 0.f;
   const float2 g = in.g;
   const float sdf = g.x;
@@ -131,7 +131,7 @@ __device__ __forceinline__ SrcOut sources_cell(const SceneDesc& S, const cfg_par
   const float fv = r1 * Yc.w / P.sootDensity;
   const float kap = P.kappaSootC * fv * Tc + P.kappaGas * Yc.z;
   const float T3 = Tc * Tc * Tc;
-  o.qrad = 4.f * kap * P.sigma * (T3 * Tc - Tamb4);
+  o.qrad = 4.f * kap * P.sigma * (T3 * Tc - R.Tamb4);
   const float dTr = o.qrad * dt / (r1 * P.cp) / (1.f + 16.f * kap * P.sigma * T3 * dt / (r1 * P.cp));
   Tc -= dTr;
   // :140-148 entrainment of ambient air through the front/back faces
@@ -215,7 +215,8 @@ __global__ void __launch_bounds__(ds_threads<TX, TY>(), TX * TY == 256 ? (NMAX =
   }
   if (threadIdx.x < 3) s_acc[threadIdx.x] = 0;
   if (threadIdx.x == blockDim.x - 1)
-    s_rcp = Rcp{__frcp_rn(P.cp), __frcp_rn(P.sO2), __frcp_rn(P.dt), __frcp_rn(P.Pr), __frcp_rn(273.15f)};
+    s_rcp = Rcp{__frcp_rn(P.cp), __frcp_rn(P.sO2), __frcp_rn(P.dt), __frcp_rn(P.Pr), __frcp_rn(273.15f),
+                SOURCES ? powf(P.Tamb, 4.f) : 0.f};
   __syncthreads();
   const Rcp R = s_rcp;
 
@@ -277,7 +278,7 @@ __global__ void __launch_bounds__(ds_threads<TX, TY>(), TX * TY == 256 ? (NMAX =
       const int r = (oj - ry0) * RW + (oi - rx0), k = oj * pc + oi;
       const float Tc = sT[cur][r]; const float4 Yc = sY[cur][r];
       if (SOURCES) {
-        const SrcOut o = sources_cell(S, P, R, in, oi, oj, Tc, Yc, powf(P.Tamb, 4.f));
+        const SrcOut o = sources_cell(S, P, R, in, oi, oj, Tc, Yc);
         S.T[k] = o.T; S.Y[k] = o.Y;
         S.SQ[k] = o.solid ? make_float2(0.f, 0.f) : make_float2(o.S, o.qrel);
         q = o.qrel; qr = o.qrad; tp = o.tpeak;
