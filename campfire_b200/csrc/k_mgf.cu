@@ -813,7 +813,7 @@ namespace {
 constexpr int CB_THREADS = 512;
 constexpr int kStagedInverseMax = 128;   // coarsest unknowns whose inverse (<= 64 KB) is staged in shared memory
 constexpr int CB_WARPS = CB_THREADS / 32;
-constexpr int SWEEP_M = 6;              // largest coarsest level of the one-warp sweeps: 12 rows per lane
+constexpr int SWEEP_M = 6;              // largest coarsest level of the one-warp sweeps: rows per lane
 constexpr int COARSEST_SCRATCH = 0;     // the coarsest keeps its stencils in registers
 using namespace mgc;
 
@@ -995,28 +995,31 @@ __device__ __forceinline__ void cb_down(const CbCtx c, int l) {
   __syncthreads();
 }
 // The 120 red-black sweeps (pressure.wgsl:132-156) in the registers of one warp, for levels up to
-// 32 cells wide: lane (g, i) owns column i of the 2 M rows from 2 M g on, as M pairs of rows with
-// one cell of each colour. A colour pass reads the other colour only: the west and east
-// neighbours by shuffles from the lanes beside (the same pair of rows), the south and north ones
-// from the lane's own registers, at the ends of its rows from the lanes below and above. Bound
-// by the latency of the 240 dependent passes: one shuffle and one cell's arithmetic each, where
-// the block's pass (coarsest_update, kept for wider levels) adds a store to shared memory, a
-// barrier and loads. A missing neighbour's coefficient is zero and a cell without open faces has
-// zeros throughout, which leaves the sums' bits as they are.
+// 64 cells wide: lane (g, k) owns columns 2k and 2k + 1 of the M rows from M g on (M even), so one
+// cell of each colour per row. A colour pass reads the other colour only: one of the west and
+// east neighbours is the lane's own cell, the other a shuffle from the lane beside, the south and
+// north ones are the lane's own rows', at the ends of its rows from the lanes below and above; which,
+// is known at compile time from the row's parity. Bound by the latency of the 240 dependent
+// passes: M + 2 shuffles and one cell's arithmetic each, where the block's pass (coarsest_update,
+// kept for the sizes that do not fit) adds a store to shared memory, a barrier and loads. A missing
+// neighbour's coefficient is zero and a cell without open faces has zeros throughout; with them
+// and without the leading +0 of pressure.wgsl:77-85 the sums keep their values.
 // Not inlined: its registers are its own, one call per coarsest solve.
-// The block of a 32x48 scene (8x12 coarsest): 31.3 -> 22.9 us, i.e. ~93 -> 58 ns per pass.
+// The block of a 32x48 scene (8x12 coarsest): 31.3 us by the block's passes, 22.8 with two shuffles
+// per cell (a column of each lane's pairs of rows), 19.8 now.
 template <int M>
-__device__ __noinline__ void sweeps_warp(float* smem, const LvO& o) {
+__device__ __noinline__ void sweeps_warp(float* smem, const LvO& o, int W) {   // W: lanes per group, (nx + 1) / 2
+  static_assert(M % 2 == 0, "a lane's first row is even");
   const LvS L = lvs_at(smem, o);
-  const int lane = threadIdx.x & 31, ng = fdiv(32, L.mnx), g = fdiv(lane, L.mnx), i = lane - g * L.nx;
+  const int lane = threadIdx.x & 31, g = lane / W, k = lane - g * W, ng = 32 / W;
   float w[2][M], e[2][M], so[2][M], no[2][M], rh[2][M], di[2][M], rc[2][M], p[2][M];
   #pragma unroll
   for (int c = 0; c < 2; c++)
     #pragma unroll
     for (int m = 0; m < M; m++) {
-      const int j = 2 * (g * M + m) + ((i + c) & 1);
+      const int i = 2 * k + ((m + c) & 1), j = g * M + m;
       w[c][m] = e[c][m] = so[c][m] = no[c][m] = rh[c][m] = di[c][m] = rc[c][m] = p[c][m] = 0.f;
-      if (g >= ng || j >= L.ny) continue;
+      if (g >= ng || i >= L.nx || j >= L.ny) continue;
       const CCell q = coarsest_cell(L, j * L.nx + i);
       if (!(q.diag > 0.f)) continue;
       if (q.hw) w[c][m] = q.w;
@@ -1025,23 +1028,23 @@ __device__ __noinline__ void sweeps_warp(float* smem, const LvO& o) {
       if (q.hn) no[c][m] = q.n;
       rh[c][m] = q.rh; di[c][m] = q.diag; rc[c][m] = q.rcp;
     }
-  const bool odd[2] = {(i & 1) != 0, (i & 1) == 0};   // colour c's cell is the upper row of its pair
   #pragma unroll 1
   for (int it = 0; it < 120; it++)
     #pragma unroll
     for (int c = 0; c < 2; c++) {
       float (&q)[M] = p[1 - c];
-      const float below = __shfl_sync(0xffffffffu, q[M - 1], lane - L.nx), above = __shfl_sync(0xffffffffu, q[0], lane + L.nx);
+      float x[M];
+      #pragma unroll
+      for (int m = 0; m < M; m++)
+        x[m] = (m + c) & 1 ? __shfl_down_sync(0xffffffffu, q[m], 1) : __shfl_up_sync(0xffffffffu, q[m], 1);
+      const float below = __shfl_sync(0xffffffffu, q[M - 1], lane - W), above = __shfl_sync(0xffffffffu, q[0], lane + W);
       #pragma unroll
       for (int m = 0; m < M; m++) {
-        const float pw = __shfl_up_sync(0xffffffffu, q[m], 1), pe = __shfl_down_sync(0xffffffffu, q[m], 1);
-        const float ps = odd[c] ? q[m] : (m > 0 ? q[m > 0 ? m - 1 : 0] : below);
-        const float pn = odd[c] ? (m < M - 1 ? q[m < M - 1 ? m + 1 : m] : above) : q[m];
-        float off = 0.f;
-        off += w[c][m] * pw;
-        off += e[c][m] * pe;
-        off += so[c][m] * ps;
-        off += no[c][m] * pn;
+        const bool right = (m + c) & 1;
+        float off = w[c][m] * (right ? q[m] : x[m]);
+        off += e[c][m] * (right ? x[m] : q[m]);
+        off += so[c][m] * (m > 0 ? q[m > 0 ? m - 1 : 0] : below);
+        off += no[c][m] * (m < M - 1 ? q[m < M - 1 ? m + 1 : m] : above);
         p[c][m] = div_by_rcp(off - rh[c][m], di[c][m], rc[c][m]);
       }
     }
@@ -1049,8 +1052,8 @@ __device__ __noinline__ void sweeps_warp(float* smem, const LvO& o) {
   for (int c = 0; c < 2; c++)
     #pragma unroll
     for (int m = 0; m < M; m++) {
-      const int j = 2 * (g * M + m) + ((i + c) & 1);
-      if (g < ng && j < L.ny) L.p[j * L.pc + i] = p[c][m];
+      const int i = 2 * k + ((m + c) & 1), j = g * M + m;
+      if (g < ng && i < L.nx && j < L.ny) L.p[j * L.pc + i] = p[c][m];
     }
 }
 // the coarsest level's solve (its p overwritten: the inverse's product, or sweeps from zero)
@@ -1107,14 +1110,13 @@ __device__ __forceinline__ void cb_coarsest(const CbCtx c) {
       const LvS L = lvs_at(smem, lvo[nl - 1]);
       const int npair = (L.nx * L.ny + 1) >> 1;
       const int nthr = (npair + 31) & ~31;
-      // pairs of rows a lane of the one-warp form owns
-      const int rows = L.nx <= 32 ? fdiv(32, L.mnx) * 2 : 0;
-      const int M = rows > 0 ? (L.ny + rows - 1) / rows : SWEEP_M + 1;
+      // rows a lane of the one-warp form owns
+      const int W = (L.nx + 1) / 2, M = W <= 32 ? (L.ny + 32 / W - 1) / (32 / W) : SWEEP_M + 1;
       if (WARP && M <= SWEEP_M) {
         if (warp == 0) {
-          if (M <= 2) sweeps_warp<2>(smem, lvo[nl - 1]);
-          else if (M <= 4) sweeps_warp<4>(smem, lvo[nl - 1]);
-          else sweeps_warp<SWEEP_M>(smem, lvo[nl - 1]);
+          if (M <= 2) sweeps_warp<2>(smem, lvo[nl - 1], W);
+          else if (M <= 4) sweeps_warp<4>(smem, lvo[nl - 1], W);
+          else sweeps_warp<SWEEP_M>(smem, lvo[nl - 1], W);
         }
       } else if ((int)threadIdx.x < nthr) {
         const CCell a = coarsest_cell(L, 2 * threadIdx.x), b = coarsest_cell(L, 2 * threadIdx.x + 1);
