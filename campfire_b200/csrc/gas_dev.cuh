@@ -134,14 +134,6 @@ __device__ __forceinline__ void loop_count(SolveCtl* ctl) {
 
 // ------------------------------------------------------------- common.wgsl
 __device__ __forceinline__ float rhoOf(const cfg_params& P, float T) { return P.rhoAmb * P.Tamb / T; }   // :33
-// :36-38 Sutherland viscosity
-__device__ __forceinline__ float muOf(const cfg_params& P, float T) {
-  return 1.716e-5f * powf(T / 273.15f, 1.5f) * (float)(273.15 + 110.4) / (T + 110.4f) * P.viscMult;
-}
-// :40-42 rho*D = k/cp
-__device__ __forceinline__ float rhoDOf(const cfg_params& P, float T) {
-  return 1.716e-5f * powf(T / 273.15f, 1.5f) * (float)(273.15 + 110.4) / (T + 110.4f) / P.Pr * P.diffMult;
-}
 __device__ __forceinline__ float4 ambY(const cfg_params& P) { return make_float4(0.f, P.YOamb, 0.f, 0.f); }  // :44
 // WGSL mix(a, b, t) = a * (1 - t) + b * t
 __device__ __forceinline__ float mixf(float a, float b, float t) { return a * (1.f - t) + b * t; }
@@ -158,24 +150,6 @@ __device__ __forceinline__ int32_t wgsl_i32_round(float v) { return __float2int_
 // Piece as laid out in the storage buffer (common.wgsl:17-23)
 struct Piece { float pos[2], angle, half, vel[2], omega, alive, Ts[4], mflux[4], charCov[4]; };
 static_assert(sizeof(Piece) == PIECE_FLOATS * 4, "Piece is 20 floats");
-
-// :47-53 signed distance to a rotated square (negative inside)
-__device__ __forceinline__ float sdBox(float px, float py, const Piece& pc) {
-  const float c = cosf(pc.angle), s = sinf(pc.angle);
-  const float dxp = px - pc.pos[0], dyp = py - pc.pos[1];
-  const float lx = c * dxp + s * dyp, ly = -s * dxp + c * dyp;
-  const float qx = fabsf(lx) - pc.half, qy = fabsf(ly) - pc.half;
-  const float mx = fmaxf(qx, 0.f), my = fmaxf(qy, 0.f);
-  return sqrtf(mx * mx + my * my) + fminf(fmaxf(qx, qy), 0.f);
-}
-// :56-62 local face index nearest to p: 0:+x 1:+y 2:-x 3:-y
-__device__ __forceinline__ uint32_t faceOf(float px, float py, const Piece& pc) {
-  const float c = cosf(pc.angle), s = sinf(pc.angle);
-  const float dxp = px - pc.pos[0], dyp = py - pc.pos[1];
-  const float lx = c * dxp + s * dyp, ly = -s * dxp + c * dyp;
-  if (fabsf(lx) > fabsf(ly)) return lx > 0.f ? 0u : 2u;
-  return ly > 0.f ? 1u : 3u;
-}
 
 // ------------------------------------------------------------- samplers (js/gpu.js:16-65)
 // at(i, j) applies the boundary rules; quad(i, j, ...) reads the 2x2 block (i..i+1, j..j+1)

@@ -23,7 +23,7 @@ struct Rcp { float cp, sO2, dt, pr, t273, Tamb4; };
 // the round trips
 struct CellIn { float2 g; float u0, u1, v0, v1, Tadv; };
 
-// rhoDOf (gas_dev.cuh) with the shared divisors' reciprocals
+// common.wgsl:40-42, rho D = k / cp (Sutherland), with the shared divisors' reciprocals
 __device__ __forceinline__ float rhoD(const cfg_params& P, const Rcp& R, float T) {
   const float v = 1.716e-5f * powf(div_by_rcp(T, 273.15f, R.t273), 1.5f) * (float)(273.15 + 110.4) / (T + 110.4f);
   return div_by_rcp(v, P.Pr, R.pr) * P.diffMult;

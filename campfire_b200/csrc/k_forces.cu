@@ -71,7 +71,7 @@ __global__ void __launch_bounds__(fr_threads<TX, TY>(), TX * TY == 256 ? 5 : 2) 
   auto u2 = [&](int i, int j) { const int k = j * pu + i; return __ldg(fxa + k) > 0.f ? __ldg(U2 + k) : 0.f; };
   auto v2 = [&](int i, int j) { const int k = j * pc + i; return __ldg(fya + k) > 0.f ? __ldg(V2 + k) : 0.f; };
   const LevelDesc L0 = S.lev[0];
-  // muOf (gas_dev.cuh)
+  // common.wgsl:36-38 Sutherland viscosity
   const float rt273 = __frcp_rn(273.15f);
   auto mu_of = [&](float t) {
     return 1.716e-5f * powf(div_by_rcp(t, 273.15f, rt273), 1.5f) * (float)(273.15 + 110.4) / (t + 110.4f) * P.viscMult;

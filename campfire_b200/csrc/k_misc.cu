@@ -135,7 +135,8 @@ __global__ void k_cfl_update(SceneDesc* scenes, int nscenes, const double* dxd, 
 // sites' arithmetic, 3 sites x the pieces that are left. 22.1 -> 8.4 us
 // at 224x320 with 16 pieces, 82 -> 10.4 us at 352x512 with 40.
 namespace {
-// sdBox and faceOf (gas_dev.cuh) with the rotation's cosine and sine at hand
+// common.wgsl:47-62, the signed distance to a rotated square (negative inside) and its nearest face
+// (0: +x, 1: +y, 2: -x, 3: -y), with the rotation's cosine and sine at hand
 struct RotPiece { float x, y, half, c, s; int n; };
 __device__ __forceinline__ float sd_rot(float px, float py, const RotPiece& q, float& lx, float& ly) {
   const float dxp = px - q.x, dyp = py - q.y;

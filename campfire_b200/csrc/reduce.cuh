@@ -68,29 +68,6 @@ __device__ __forceinline__ bool scene_reduce(const SceneDesc& S, int tile, int n
   return true;
 }
 
-// Two sums at once (partials at part[2 tile], part[2 tile + 1]); same protocol.
-__device__ __forceinline__ bool scene_reduce2(const SceneDesc& S, int tile, int ntiles, double a, double b,
-                                              double* sh, double* ta, double* tb) {
-  __shared__ int s_last2;
-  if (threadIdx.x == 0) {
-    S.part[2 * tile] = a;
-    S.part[2 * tile + 1] = b;
-    const unsigned prev = arrive_acq_rel(&S.solve->counter);
-    s_last2 = (prev == (unsigned)ntiles - 1u) ? 1 : 0;
-  }
-  __syncthreads();
-  if (!s_last2) return false;
-  double va = 0.0, vb = 0.0;
-  for (int k = threadIdx.x; k < ntiles; k += blockDim.x) {
-    va += __ldcg(S.part + 2 * k);
-    vb += __ldcg(S.part + 2 * k + 1);
-  }
-  const double sa = block_sum(va, sh);
-  const double sb = block_sum(vb, sh);
-  if (threadIdx.x == 0) { *ta = sa; *tb = sb; S.solve->counter = 0u; }
-  return true;
-}
-
 // Three sums at once (partials at part[3 tile + 0..2]); same protocol.
 __device__ __forceinline__ bool scene_reduce3(const SceneDesc& S, int tile, int ntiles, double a, double b, double c,
                                               double* sh, double* ta, double* tb, double* tc) {
