@@ -262,6 +262,14 @@ __device__ __forceinline__ float div_tiny(float x, float d, float r) {
   return x != 0.f && fabsf(x) < 1e-30f ? x / d : div_by_rcp(x, d, r);
 }
 
+// x / d from r = RN(1/d) in FP64: Markstein's correction twice, so that the first quotient need not
+// be within an ulp; the IEEE quotient for quotients and residuals in the normal range
+__device__ __forceinline__ double ddiv_by_rcp(double x, double d, double r) {
+  double q = __dmul_rn(x, r);
+  q = __fma_rn(__fma_rn(-q, d, x), r, q);
+  return __fma_rn(__fma_rn(-q, d, x), r, q);
+}
+
 // advect.wgsl:28-34: vel = (s_U, s_V)/dx; RK2 midpoint back-trace (dt < 0 traces forward).
 // The quotient by dx from rdx = RN(1/dx): the IEEE one, except that a velocity of -0 comes
 // out +0, which moves no trace point (g - h * (+-0) = g)

@@ -14,13 +14,6 @@
 
 namespace cfg {
 
-// x / d from r = RN(1/d) in FP64: Markstein's correction twice, so that the first quotient need not
-// be within an ulp; the IEEE quotient for quotients and residuals in the normal range
-__device__ __forceinline__ double ddiv_by_rcp(double x, double d, double r) {
-  double q = __dmul_rn(x, r);
-  q = __fma_rn(__fma_rn(-q, d, x), r, q);
-  return __fma_rn(__fma_rn(-q, d, x), r, q);
-}
 // reciprocals of the divisors every face and cell shares, once per CTA
 struct FRcp { float t273, tamb, depth, rT, dx, dt; double ddx, ddt; };
 
