@@ -197,6 +197,12 @@ int Engine::init(int device, int n, const int* nx, const int* ny, const double* 
   CFG_CUDA(cudaMalloc(&d_dxd_, sizeof(double) * n));
   CFG_CUDA(cudaMalloc(&d_alpha_, sizeof(double) * n));
   for (int s = 0; s < n; s++) CFG_TRY(alloc_scene(scenes_[s]));
+  // Many waves of tiles (several scenes): advection takes 32x16 cells, whose halo is a smaller share.
+  // 64 uneven scenes (13854 tiles of 32x8) 3775 -> 3714 us per step; one scene of 512x768 (1536 tiles, 3.5
+  // waves) 728 -> 735: 32x8.
+  long adv = 0;
+  for (const Scene& sc : scenes_) adv += (long)((sc.nx + 31) / 32) * ((sc.ny + 7) / 8);
+  if (adv > kManyAdvectTiles) tiles_[TK_ADVECT] = 2;
   CFG_TRY(build_worklists());
   for (int s = 0; s < n; s++) {
     scenes_[s].desc.solve = d_solve_ + s;

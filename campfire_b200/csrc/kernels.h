@@ -36,6 +36,7 @@ enum TmapKind { TM_P = 0, TM_PB, TM_RHS, TM_AX, TM_AY, TM_PC, TM_PER_LEVEL };
 constexpr int TMAP_BYTES = 128;
 constexpr int COARSE_CELLS = 6144;                   // default: largest level handled by the one-CTA coarse block
 constexpr int kBlockCells = 2048;                    // the block starts no earlier than a level of this size (Engine::choose_lc)
+constexpr int kManyAdvectTiles = 4096;               // 32x8 tiles of all scenes from which advection's default is 32x16 (Engine::init)
 constexpr int kUnrolledCycles = 12;                  // cycles laid out ahead of the step graph's loop, at most
 constexpr size_t kCoarseSmemMax = 232448 - 2048;     // dynamic shared memory of the coarse block (227 KB less static)
 constexpr int PR_TX = 32, PR_TY = 8;                 // projection

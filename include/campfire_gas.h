@@ -261,7 +261,8 @@ int cfg_autotune(int device, int nscenes, const int* nx, const int* ny, int coar
                  int* best_cells, int* cand_cells, double* cand_ms, int* ncand);
 
 /* Tile shapes of the advection, diffusion + sources and forces kernels (no counterpart in the
- * reference, whose workgroups are 8x8): 0 = 32x8 cells (default), 1 = 64x8, 2 = 32x16. Every
+ * reference, whose workgroups are 8x8): 0 = 32x8 cells (default; advection of an engine with more
+ * than 4096 such tiles: 2), 1 = 64x8, 2 = 32x16. Every
  * shape gives the same bits; only the time changes. Batch views: use cfg_batch_set_tiles. */
 int cfg_set_tiles(cfg_sim* sim, int advect, int diffuse_sources, int forces);
 int cfg_batch_set_tiles(cfg_batch* b, int advect, int diffuse_sources, int forces);

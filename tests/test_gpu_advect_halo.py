@@ -33,3 +33,19 @@ def test_advection_bits_over_displacements(oracle_mod, nx, ny, cells):
         for f in ("T2", "Y2", "U2", "V2"):
             assert np.array_equal(g.readBuffer(f), o.read(f).astype(np.float32)), (shape, f)
         g.close()
+
+
+@pytest.mark.parametrize("n", [10, 11])
+def test_many_tiles_take_the_larger_ones(n):
+    # 3840 and 4224 tiles of 32x8 cells: the default shape on either side of its line gives shape 0's bits
+    out = []
+    for explicit in (False, True):
+        b = cb.Batch([(256, 384)] * n, 0.8, [0.002] * n)
+        for k in (0, n - 1):
+            load_scene(b.scenes[k], cb.generate_scene(0, 256, 384, 0.8, 3 + k))
+        if explicit:
+            b.set_tiles(0, 0, 0)
+        b.step(1); b.synchronize()
+        out.append([b.scenes[k].readBuffer(f) for k in (0, n - 1) for f in ("T", "Y", "U", "V")])
+        b.close()
+    assert all(np.array_equal(x, y) for x, y in zip(*out))
