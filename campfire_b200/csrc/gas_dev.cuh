@@ -215,8 +215,8 @@ struct VField {
 // floor(x) as an integer and the fraction x - floor(x): x + 1.5 2^23 rounded down has an ulp of 1 for
 // |x| < 2^22, so its low bits hold the floor and subtracting the constant again gives it as a
 // float, exactly; three full-rate operations where floorf and the conversion take two of a
-// sixteenth. Beyond that range (or for a NaN) the integer lies outside every grid, where the
-// samplers read the boundary values.
+// sixteenth. Trace points stay within that range (VelSampler::moved); for a NaN the integer lies outside
+// every grid.
 __device__ __forceinline__ int floor_frac(float x, float& frac) {
   const float y = __fadd_rd(x, 12582912.f);
   frac = x - (y - 12582912.f);
@@ -275,6 +275,14 @@ __device__ __forceinline__ double ddiv_by_rcp(double x, double d, double r) {
 // out +0, which moves no trace point (g - h * (+-0) = g)
 struct VelSampler {
   UField u; VField v; float dx, rdx;
+  // g moved back by d cells, at most 4 million (a NaN kept): points beyond that lie outside every grid (16384
+  // cells at most), where the samplers read boundary values that do not depend on the distance, and
+  // floor_frac's range ends at 2^22
+  static __device__ __forceinline__ float moved(float g, float d) {
+    float m;
+    asm("min.NaN.xorsign.abs.f32 %0, %1, %2;" : "=f"(m) : "f"(d), "f"(4e6f));
+    return g - m;
+  }
   __device__ __forceinline__ void vel(float gx, float gy, float& vx, float& vy) const {
     vx = div_by_rcp(sample(u, gx, gy, 0.f, 0.5f), dx, rdx);
     vy = div_by_rcp(sample(v, gx, gy, 0.5f, 0.f), dx, rdx);
@@ -282,9 +290,9 @@ struct VelSampler {
   __device__ __forceinline__ void trace(float gx, float gy, float tdt, float& ox, float& oy) const {
     float vx, vy; vel(gx, gy, vx, vy);
     const float hd = 0.5f * tdt;
-    const float mx = gx - hd * vx, my = gy - hd * vy;
+    const float mx = moved(gx, hd * vx), my = moved(gy, hd * vy);
     vel(mx, my, vx, vy);
-    ox = gx - tdt * vx; oy = gy - tdt * vy;
+    ox = moved(gx, tdt * vx); oy = moved(gy, tdt * vy);
   }
 };
 

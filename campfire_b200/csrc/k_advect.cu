@@ -155,8 +155,8 @@ __device__ __forceinline__ void vel_vface(const VelSampler& s, int i, int j, flo
 __device__ __forceinline__ void trace_from(const VelSampler& s, float gx, float gy, float vx, float vy, float tdt,
                                            float& ox, float& oy) {
   const float hd = 0.5f * tdt;
-  float wx, wy; s.vel(gx - hd * vx, gy - hd * vy, wx, wy);
-  ox = gx - tdt * wx; oy = gy - tdt * wy;
+  float wx, wy; s.vel(s.moved(gx, hd * vx), s.moved(gy, hd * vy), wx, wy);
+  ox = s.moved(gx, tdt * wx); oy = s.moved(gy, tdt * wy);
 }
 // sample and the corners' range at one point
 template <class F>
