@@ -19,6 +19,10 @@ namespace {
 // IEEE ones) and powf(Tamb, 4)
 struct Rcp { float cp, sO2, dt, pr, t273, Tamb4; };
 
+// The coefficient of a closed face, a value no open one has (f rho D is +0 at least, or a NaN, which reaches the
+// cells on both sides as in diffuse.wgsl)
+constexpr float kClosed = -0.f;
+
 // what the sources read beside the diffused state; loaded before the diffusion, whose work covers
 // the round trips
 struct CellIn { float2 g; float u0, u1, v0, v1, Tadv; };
@@ -234,11 +238,11 @@ __global__ void __launch_bounds__(ds_threads<TX, TY>(), TX * TY == 256 ? (NMAX =
       if (i < xa || i > xb || j < ya || j > yb) continue;
       if (j < yb) {
         const float f = i > 0 && i < nx ? __ldg(S.fx + j * pu + i) : 0.f;
-        sAx[r] = f > 0.f ? f * rhoD(P, R, 0.5f * (Ti[r] + Ti[r - 1])) : 0.f;
+        sAx[r] = f > 0.f ? f * rhoD(P, R, 0.5f * (Ti[r] + Ti[r - 1])) : kClosed;
       }
       if (i < xb) {
         const float f = j > 0 && j < ny ? __ldg(S.fy + j * pc + i) : 0.f;
-        sAy[r] = f > 0.f ? f * rhoD(P, R, 0.5f * (Ti[r] + Ti[r - RW])) : 0.f;
+        sAy[r] = f > 0.f ? f * rhoD(P, R, 0.5f * (Ti[r] + Ti[r - RW])) : kClosed;
       }
     }
     __syncthreads();
@@ -247,11 +251,11 @@ __global__ void __launch_bounds__(ds_threads<TX, TY>(), TX * TY == 256 ? (NMAX =
       if (i < xa || i >= xb || j < ya || j >= yb) continue;
       const float T0 = Ti[r]; const float4 Y0 = Yi[r];
       float sTa = 0.f; float sYx = 0.f, sYy = 0.f, sYz = 0.f;
-      // west, east, south, north; a closed face's coefficient is zero
+      // west, east, south, north
       #define CFG_DIFF_FACE(coef, roff)                                         \
         {                                                                       \
           const float a = (coef);                                               \
-          if (a > 0.f) {                                                        \
+          if (__float_as_uint(a) != __float_as_uint(kClosed)) {                 \
             const float Tn = Ti[r + (roff)]; const float4 Yn = Yi[r + (roff)];  \
             sTa += a * (Tn - T0);                                               \
             sYx += a * (Yn.x - Y0.x); sYy += a * (Yn.y - Y0.y); sYz += a * (Yn.z - Y0.z); \
