@@ -414,10 +414,11 @@ __global__ void __launch_bounds__(RAD_THREADS) k_radiation(const SceneDesc* __re
             float hx, hy; hitBox(ox, oy, ddx, ddy, pc, sc[n], ss[n], hx, hy);
             if (hx > 0.f && hx < tHit) { tHit = hx; hitT = pc.Ts[(uint32_t)hy]; hitN = n; }
           }
-        const unsigned mask = __activemask();
+        // whole warps are here (RT G is a multiple of 32 for every power of two of rays): the full mask brings
+        // the lanes together again that left the loop over the pieces at different turns
         for (int o = G / 2; o > 0; o >>= 1) {
-          const float t2 = __shfl_xor_sync(mask, tHit, o), T2 = __shfl_xor_sync(mask, hitT, o);
-          const int n2 = __shfl_xor_sync(mask, hitN, o);
+          const float t2 = __shfl_xor_sync(0xffffffffu, tHit, o), T2 = __shfl_xor_sync(0xffffffffu, hitT, o);
+          const int n2 = __shfl_xor_sync(0xffffffffu, hitN, o);
           if (t2 < tHit || (t2 == tHit && n2 < hitN)) { tHit = t2; hitT = T2; hitN = n2; }
         }
         if (g == 0) {
