@@ -389,8 +389,13 @@ int Engine::checkpoint_save(int s, const char* path) {
   for (auto& it : sc.items) {
     if (!ok) break;
     if (!it.state) continue;
-    buf.resize(it.bytes);
-    CFG_CUDA(cudaMemcpy(buf.data(), it.ptr, it.bytes, cudaMemcpyDeviceToHost));
+    // the spare species array holds what reads and the radiation pass left there: zeros in the file
+    if (it.ptr == sc.desc.Yw) {
+      buf.assign(it.bytes, 0);
+    } else {
+      buf.resize(it.bytes);
+      CFG_CUDA(cudaMemcpy(buf.data(), it.ptr, it.bytes, cudaMemcpyDeviceToHost));
+    }
     const uint64_t n = it.bytes;
     ok = put(&n, 8) && put(buf.data(), it.bytes);
   }
