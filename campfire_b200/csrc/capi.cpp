@@ -258,7 +258,6 @@ extern "C" int cfg_autotune(int device, int nscenes, const int* nx, const int* n
   return guarded([&] {
     std::vector<double> width(nscenes, 0.8), dt(nscenes, 0.002);
     cfg::Engine eng;
-    eng.uncap_block();
     CFG_TRY(eng.init(device, nscenes, nx, ny, width.data(), dt.data()));
     for (int s = 0; s < nscenes; s++) CFG_TRY(cfg::load_generated_scene(eng, s, 0, 0.8, 1234 + s));
     if (coarse_direct) {
@@ -281,8 +280,16 @@ extern "C" int cfg_autotune(int device, int nscenes, const int* nx, const int* n
     int k = 0;
     double best = 1e300;
     *best_cells = 0;
-    for (int c : cells) {
+    std::vector<int> at, next, w;
+    for (size_t q = 0; q < cells.size(); q++) {
+      const int c = cells[q];
       if (k >= *ncand) break;
+      // thresholds that start every scene's block at the same level are one schedule: the smallest stands for it
+      if (q + 1 < cells.size()) {
+        eng.block_starts(c, at, w);
+        eng.block_starts(cells[q + 1], next, w);
+        if (at == next) continue;
+      }
       if (eng.set_coarse_cells(c) != CFG_OK) continue;   // does not fit in shared memory
       double ms = 0, bytes = 0, per = 0;
       CFG_TRY(eng.time_kernel("vcycle", iters, &ms, &bytes, &per));

@@ -120,9 +120,12 @@ int Engine::activate() const {
 // arrays fit in one CTA's shared memory (else at the coarsest level), or later: `cap` cells at
 // most (level 0, which a block may cover whole, only where `cap0`). Every start gives the same
 // pressures; above kBlockCells the tiled kernels of a level are the faster ones, ~7 us down and
-// up against 12-17 us on one SM (per step: 128x192 in FP32 cycles 344 -> 268 us with 64x96 tiled,
-// 224x320 126 -> 113 with 56x80 tiled; 1536 to 4600 cells differ by under 2%). In the FP64
-// modes a block that covers level 0 stays: the loop's update follows from it.
+// up against 12-17 us on one SM. Whole steps with a request of 6144 cells, uncapped and capped: one
+// scene, one fixed cycle, 64x96 91 and 72 us, 224x320 100 and 85, 512x768 226 and 206; to 1e-4
+// 128x192 467 and 338; FP64 to 1e-6 256x384 485 and 331. Batches, FP64 to 1e-6: 8 of 256x384 1195
+// and 1023, 24 uneven 1484 and 1398, 64 uneven 3357 and 3311 (one fixed cycle 942 and 936), 64 of
+// 128x192 1867 and 1757; none was faster uncapped. In the FP64 modes a block that covers level 0
+// stays: the loop's update follows from it.
 // cs > 0: the cluster coarse phase, which starts at level 1 at the earliest (level 0
 // always runs as tiled kernels) and fits each CTA's share of the levels
 int Engine::choose_lc(const Scene& sc, int cells, int cs, int cap, bool cap0) {
@@ -160,7 +163,7 @@ int Engine::init(int device, int n, const int* nx, const int* ny, const double* 
     }
     sc.nlev = L;
     if (sc.lnx[L - 1] * sc.lny[L - 1] > 256) return fail(CFG_ERR_RANGE, "coarsest level too large");
-    sc.lc = choose_lc(sc, coarse_cells_, 0, block_cap_, true);
+    sc.lc = choose_lc(sc, coarse_cells_, 0, kBlockCells, true);
     coarse_smem_ = std::max(coarse_smem_, coarse_smem_bytes(sc.lnx, sc.lny, sc.lc, sc.nlev));
     const int cn = sc.lnx[L - 1] * sc.lny[L - 1], cbw = sc.lnx[L - 1];
     if (cbw <= 32) { cf_smem_ = std::max(cf_smem_, coarse_factor_smem(cn)); cf_bw_ = std::max(cf_bw_, cbw); }
@@ -527,14 +530,9 @@ int Engine::set_coarse_cluster(int cs) {
   return rc;
 }
 
-int Engine::set_coarse_cells(int cells) {
-  if (cells < 1) return fail(CFG_ERR_INVAL, "coarse cells must be >= 1");
-  CFG_TRY(activate());
-  CFG_CUDA(cudaStreamSynchronize(st()));
-  const int cs = coarse_cluster_;
-  if (cs > 0 && w_cells_ > 0) return fail(CFG_ERR_INVAL, "the W tail runs in the one-CTA coarse block only");
-  size_t smem = 0;
-  std::vector<int> lcs(scenes_.size()), lws(scenes_.size());
+void Engine::block_starts(int cells, std::vector<int>& lcs, std::vector<int>& lws) const {
+  lcs.resize(scenes_.size());
+  lws.resize(scenes_.size());
   for (size_t s = 0; s < scenes_.size(); s++) {
     const Scene& sc = scenes_[s];
     // the W tail: level nlev - 3 (two above the coarsest) visits level nlev - 2 twice when it has
@@ -543,8 +541,22 @@ int Engine::set_coarse_cells(int cells) {
     if (w_cells_ > 0 && sc.nlev >= 3 && sc.lnx[sc.nlev - 3] * sc.lny[sc.nlev - 3] <= w_cells_) lw = sc.nlev - 3;
     lws[s] = lw;
     const int lwc = lw < sc.nlev ? sc.lnx[lw] * sc.lny[lw] : 0;
-    lcs[s] = choose_lc(sc, std::max(cells, lwc), cs, std::max(block_cap_, lwc), !any_fp64());
-    if (lw < sc.nlev && lcs[s] > lw)
+    lcs[s] = choose_lc(sc, std::max(cells, lwc), coarse_cluster_, std::max(kBlockCells, lwc), !any_fp64());
+  }
+}
+
+int Engine::set_coarse_cells(int cells) {
+  if (cells < 1) return fail(CFG_ERR_INVAL, "coarse cells must be >= 1");
+  CFG_TRY(activate());
+  CFG_CUDA(cudaStreamSynchronize(st()));
+  const int cs = coarse_cluster_;
+  if (cs > 0 && w_cells_ > 0) return fail(CFG_ERR_INVAL, "the W tail runs in the one-CTA coarse block only");
+  size_t smem = 0;
+  std::vector<int> lcs, lws;
+  block_starts(cells, lcs, lws);
+  for (size_t s = 0; s < scenes_.size(); s++) {
+    const Scene& sc = scenes_[s];
+    if (lws[s] < sc.nlev && lcs[s] > lws[s])
       return fail(CFG_ERR_RANGE, "the W tail's levels do not fit in the coarse block's shared memory");
     smem = std::max(smem, cs > 0 ? cluster_smem_bytes(sc.lnx, sc.lny, lcs[s], sc.nlev, cs)
                                  : coarse_smem_bytes(sc.lnx, sc.lny, lcs[s], sc.nlev));
@@ -1201,7 +1213,7 @@ int Engine::set_solver(int mode, int ncycles, double tol, int max_cycles) {
   // a block that may cover level 0 in one kind of mode only
   if (any_fp64() != was && coarse_cluster_ == 0)
     for (const Scene& sc : scenes_)
-      if (sc.nx * sc.ny > block_cap_ && sc.nx * sc.ny <= coarse_cells_) { CFG_TRY(set_coarse_cells(coarse_cells_)); break; }
+      if (sc.nx * sc.ny > kBlockCells && sc.nx * sc.ny <= coarse_cells_) { CFG_TRY(set_coarse_cells(coarse_cells_)); break; }
   return upload_ctl();
 }
 

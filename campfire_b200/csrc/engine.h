@@ -164,7 +164,8 @@ class Engine {
   // most `cells` cells (levels above it run as tiled down/up kernels)
   int set_coarse_cells(int cells);
   int coarse_cells() const { return coarse_cells_; }
-  void uncap_block() { block_cap_ = 1 << 30; }   // the autotuner times every start as asked
+  // each scene's first level of the coarse block, and of its W tail, for that request
+  void block_starts(int cells, std::vector<int>& lcs, std::vector<int>& lws) const;
   // cycle shape of the pressure loop: with cells > 0, the level two above the coarsest visits
   // its coarser level twice per cycle (the W tail) when it has at most `cells` cells; that
   // level always runs inside the one-CTA coarse block
@@ -280,7 +281,6 @@ class Engine {
   size_t cluster_smem_ = 0;
   int cf_bw_ = 0;               // the widest coarsest level (k_coarse_factor's register window)
   int coarse_cells_ = COARSE_CELLS;
-  int block_cap_ = kBlockCells;
   bool graph_loops_ = true;   // the step graph holds the pressure loop's WHILE node
   int w_cells_ = 0;             // set_coarse_w
   int coarse_direct_ = 0;

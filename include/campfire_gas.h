@@ -205,7 +205,7 @@ int cfg_time_kernel(cfg_sim* sim, const char* kernel, int iters, double* mean_ms
  * scene, the levels above as tiled down/up kernels. Results are bit-identical for every
  * choice; only the time changes, and levels above 2048 cells, on which the tiled kernels are
  * faster, run tiled whatever the choice (in the FP64 modes a block that covers level 0 stays
- * whole). Default 6144. Batch views: use cfg_batch_set_coarse_cells. */
+ * whole, and a W tail's level stays in the block). Default 6144. Batch views: use cfg_batch_set_coarse_cells. */
 int cfg_set_coarse_cells(cfg_sim* sim, int cells);
 /* Where that coarse phase runs: 0 (default) one CTA per scene; 2, 4, 8 or 16: a thread-block
  * cluster of that many CTAs per scene, each owning a share of every level's rows (from level 1
@@ -254,7 +254,9 @@ int cfg_batch_krylov_folded(cfg_batch* b, int* folded);
 /* Autotuner of that schedule (no counterpart in the reference): builds a scratch batch of
  * these sizes on `device` with generated scenes, runs one step to build the coefficients
  * (and, with coarse_direct, the coarsest inverse), then times `iters` fused V-cycles for
- * every threshold that fits (the level sizes). On entry *ncand is the capacity of
+ * every threshold that fits and gives a schedule of its own (the level sizes; of several that
+ * start every scene's block at the same level, as those above 2048 cells may, the smallest).
+ * On entry *ncand is the capacity of
  * cand_cells/cand_ms; on return, the candidates timed (ms per cycle) and *best_cells the
  * fastest. */
 int cfg_autotune(int device, int nscenes, const int* nx, const int* ny, int coarse_direct, int iters,
