@@ -200,9 +200,12 @@ int Engine::init(int device, int n, const int* nx, const int* ny, const double* 
   CFG_CUDA(cudaMalloc(&d_dxd_, sizeof(double) * n));
   CFG_CUDA(cudaMalloc(&d_alpha_, sizeof(double) * n));
   for (int s = 0; s < n; s++) CFG_TRY(alloc_scene(scenes_[s]));
-  // Many waves of tiles (several scenes): advection takes 32x16 cells, whose halo is a smaller share.
-  // 64 uneven scenes (13854 tiles of 32x8) 3775 -> 3714 us per step; one scene of 512x768 (1536 tiles, 3.5
-  // waves) 728 -> 735: 32x8.
+  // Many waves of tiles (several scenes; one scene has at most 4096): advection takes 32x16 cells, whose
+  // halo is a smaller share. Us per step of one fixed cycle with 32x8 and 32x16: 4 uneven scenes (750 tiles
+  // of 32x8) 121 and 123, 4 of 256x384 (1536) 177 and 176, 12 uneven (2250) 229 and 225, 11 of 256x384
+  // (4224) 377 and 366, 24 uneven (4500) 405 and 392, 48 uneven (9000) 758 and 719; one scene of 512x768
+  // (1536) 178 and 178, to 1e-10 728 and 735. The line lies where the gain is 3% and no longer depends
+  // on the sizes.
   long adv = 0;
   for (const Scene& sc : scenes_) adv += (long)((sc.nx + 31) / 32) * ((sc.ny + 7) / 8);
   if (adv > kManyAdvectTiles) tiles_[TK_ADVECT] = 2;
@@ -1475,10 +1478,16 @@ int Engine::ensure_graph() {
   cudaError_t e = cudaStreamGetCaptureInfo(s, &status, nullptr, &g, nullptr, nullptr);
   if (e != cudaSuccess) return abort_capture(e, "cudaStreamGetCaptureInfo");
   // The first cycles are laid out one after the other, up to kUnrolledCycles: all of a fixed count, or
-  // one per decade of the asked tolerance (what the solves need or a little less: 5-6 for 1e-6,
-  // 9-11 for 1e-10). Only what remains is a WHILE node, which costs a step ~10 us to enter and 5 us
-  // between two cycles (256x384: 48 us per looped cycle, 43 per laid-out one) where a laid-out cycle
-  // after the last needed one costs 8 us (512x768: 13), its kernels leaving on the scene's flag.
+  // one per decade of the asked tolerance (burning scenes need that or more: 5-8 for 1e-6, 9-18 for
+  // 1e-10; smooth plumes 4 and 7). Only what remains is a WHILE node, which costs a step ~10 us to
+  // enter and 5 us between two cycles (256x384: 48 us per looped cycle, 43 per laid-out one) where a
+  // laid-out cycle after the last needed one costs 8 us (512x768: 13), its kernels leaving on the
+  // scene's flag. Us per step with the loop alone and with cycles laid out: 256x384 to 1e-6 burning
+  // 328 and 304, plume 207 and 209; to 1e-10 585 and 542, 336 and 326; 512x768 to 1e-10 922 and 875,
+  // 615 and 611; 24 uneven scenes to 1e-10 1830 and 1805, 1179 and 1202. Gas at rest, whose solves need
+  // no cycle, is what loses: 87 and 118 (256x384, 1e-6), 191 and 318 (512x768, 1e-10). Eight laid-out
+  // cycles at most gave the last 288 and a plume to 1e-10 5% less, but every burning step to 1e-10 1-2%
+  // more; six, or turns of two cycles, 2-3% more.
   const bool fixed = mode_ == CFG_SOLVE_FIXED;
   const int wanted = fixed ? ncycles_ : (int)std::lround(-std::log10(tol_));
   const int ahead = coarse_cluster_ > 0 ? 0 : std::min(std::max(std::min(wanted, fixed ? ncycles_ : max_cycles_), 0), kUnrolledCycles);

@@ -4,9 +4,9 @@
 // The first-order values Th, Yh, Uh, Vh (advect.wgsl:68-76, 36-47) exist only
 // in shared memory: each CTA computes them on its tile plus a halo of H cells,
 // then applies the MacCormack correction (:78-103, :49-66) to its own cells and
-// faces. A forward-trace sample that lands outside the halo (a displacement of
-// H cells or more) recomputes the first-order value from global memory, so the
-// result does not depend on the time step. Global traffic per cell: U, V, T, Y
+// faces. A forward-trace sample that lands outside the staged halo (at most H
+// cells wide) recomputes the first-order value from global memory, so the
+// result depends on neither the time step nor the tile. Global traffic per cell: U, V, T, Y
 // read (through L1), T2, Y2, U2, V2 written; the 40 bytes/cell of Th/Yh and
 // 8 bytes/face of Uh/Vh of the reference schedule never reach HBM.
 #include "gas_dev.cuh"

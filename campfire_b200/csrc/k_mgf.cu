@@ -4,8 +4,9 @@
 // Each fine level l < lc is handled by two kernels per cycle:
 //   down: stage p, rhs, ax, ay of the tile plus a 5-cell halo into shared
 //         memory with TMA tensor copies, run the 4 colour passes (red, black,
-//         red, black), each one cell narrower than the last, then the residual
-//         of the tile's cells and its restriction to the coarse rhs (coarse p = 0);
+//         red, black), each over the whole region and exact one cell further
+//         in than the last, then the residual of the tile's cells and its
+//         restriction to the coarse rhs (coarse p = 0);
 //   up:   the same staging (and the coarse p under the tile), bilinear
 //         prolongation of the coarse correction, 4 colour passes (black, red,
 //         black, red); on level 0 also the residual norm (FP32 modes) or
@@ -17,7 +18,8 @@
 // Levels lc..coarsest run in one CTA per scene (coarse block): every level's
 // arrays staged into shared memory by TMA bulk copies, __syncthreads between
 // passes, and the coarsest level's 120 red-black sweeps (pressure.wgsl:132-156)
-// on one thread per red/black cell pair with a named barrier.
+// in one warp's registers (levels that do not fit there: on one thread per
+// red/black cell pair with a named barrier).
 #include "gas_dev.cuh"
 #include "kernels.h"
 #include "reduce.cuh"
@@ -94,12 +96,13 @@ __device__ __forceinline__ bool scene_idle(const SolveState* ss) { return *(cons
 // before the wait, with the state copies' tensor maps prefetched; else after it, with
 // stage_state, once the scene's flag says it still cycles): one thread initialises both barriers and requests the coefficients
 // ax, ay on bar[0]; they are built before the pressure loop and written by no loop kernel
-// (the loop is entered through a full dependency: a graph node or a memset). stage_state
+// (the first cycle's first kernel starts once the kernels that build them have completed: it is
+// launched without programmatic dependence, or is a loop body's first node). stage_state
 // (after the wait): p from map `pkind`, rhs and the coarse p under the tile on bar[1]; with
 // `copy` false nothing is requested and bar[1] completes on its arrival; with `pload` false p
-// is not copied (the caller zero-fills its box). The copies are
-// issued whether or not the scene still cycles, so the read of its `active` flag overlaps
-// them. tile_wait: all threads wait for one barrier (bounded); false in every thread if a
+// is not copied (the caller zero-fills its box). With one scene the copies are issued before
+// its `active` flag is read again, which then overlaps them; with several once the flag says
+// that the scene cycles. tile_wait: all threads wait for one barrier (bounded); false in every thread if a
 // wait ran out, after recording the error and waiting once more for the copies in flight.
 __device__ __forceinline__ void stage_coef(const SceneDesc& S, int level, const Tile& t, uint64_t* bar) {
   if (threadIdx.x == 0) {

@@ -319,14 +319,13 @@ __device__ float4 fragment(const RenderIn& in, float wx, float wy, float uvy) {
 
 }  // namespace
 
-// Persistent CTAs over 16x16-pixel tiles. Bound by FP32 issue and the special-function pipe: a gas
-// pixel evaluates two exponentials per wavelength. The wavelengths' own values, the firelight
+// Persistent CTAs over 16x16-pixel tiles. Bound by instruction issue: a lit gas pixel evaluates 12
+// wavelengths of two exponentials each. The wavelengths' own values, the firelight
 // spectrum and the pieces' rotations are set up once per CTA instead of per pixel (~200 of the
 // ~230 exponentials of a gas pixel were the matching functions of 12 fixed wavelengths), and each
-// warp first finds which pieces reach its 16x2 pixels. 734x1080 photo of
-// 224x320 with 16 pieces: 252 -> 45 us (the image kernel alone 50 us
-// at 734x1080 of a burning fire); 1468x2160 of 352x512 with 40 pieces: 1170 -> 170 us. Bound by
-// instruction issue: 12 exponentials and radiances per lit pixel.
+// warp first finds which pieces reach its 16x2 pixels. 734x1080 photo of 224x320 with 16 pieces:
+// 252 -> 45 us (50 us in a frame of a burning fire, which lights more pixels); 1468x2160 of 352x512
+// with 40 pieces: 1170 -> 170 us.
 __global__ void __launch_bounds__(256) k_render(const SceneDesc* __restrict__ scenes, int scene, cfg_render_params R,
                                                 const float4* __restrict__ wood, int W, int H, float4* __restrict__ out) {
   __shared__ Wave tab[NL];

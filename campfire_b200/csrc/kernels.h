@@ -113,7 +113,9 @@ void launch_pack(uint32_t* dst, const void* src, size_t pitch, int w, int h, cud
 // scene for levels lc..coarsest
 // count_iter: the kernel opens a graph loop iteration (loop_count); pcg: level 0 of the
 // fused Krylov mode (applies the previous cycle's update); nscenes: the engine's scenes
-// (with one, tiles are requested before the scene's active flag is read: it only stops the loop)
+// (with one, a tile's coefficients are requested before the wait on the previous kernel, unless the
+// scene's flag has fallen by then, and its state before the flag is read again); pdl: the kernel may
+// start before its predecessor has completed
 void launch_mg_down(const SceneDesc* scenes, int nscenes, const Work* work, int ntiles, int level, SolveCtl* ctl,
                     int count_iter, int pcg, bool pdl, cudaStream_t st);
 void launch_mg_up(const SceneDesc* scenes, int nscenes, const Work* work, int ntiles, int level, int tail, SolveCtl* ctl,
