@@ -278,11 +278,12 @@ struct VelSampler {
   // g moved back by d cells, at most 4 million (a NaN kept): points beyond that lie outside every grid (16384
   // cells at most), where the samplers read boundary values that do not depend on the distance, and
   // floor_frac's range ends at 2^22
-  static __device__ __forceinline__ float moved(float g, float d) {
+  static __device__ __forceinline__ float bounded(float d) {
     float m;
     asm("min.NaN.xorsign.abs.f32 %0, %1, %2;" : "=f"(m) : "f"(d), "f"(4e6f));
-    return g - m;
+    return m;
   }
+  static __device__ __forceinline__ float moved(float g, float d) { return g - bounded(d); }
   __device__ __forceinline__ void vel(float gx, float gy, float& vx, float& vy) const {
     vx = div_by_rcp(sample(u, gx, gy, 0.f, 0.5f), dx, rdx);
     vy = div_by_rcp(sample(v, gx, gy, 0.5f, 0.f), dx, rdx);

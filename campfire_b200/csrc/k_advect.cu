@@ -151,11 +151,11 @@ __device__ __forceinline__ void vel_vface(const VelSampler& s, int i, int j, flo
   vx = div_by_rcp(mixf(mixf(A, C, 0.5f), mixf(D, E, 0.5f), 0.5f), s.dx, s.rdx);
   vy = div_by_rcp(__ldg(s.v.a + j * s.v.pc + i), s.dx, s.rdx);
 }
-// the second half of VelSampler::trace from (gx, gy), whose velocity is (vx, vy)
-__device__ __forceinline__ void trace_from(const VelSampler& s, float gx, float gy, float vx, float vy, float tdt,
+// the second half of VelSampler::trace from (gx, gy), whose displacement in half the step is (hx, hy) (its negative
+// for the trace forward, with -dt)
+__device__ __forceinline__ void trace_from(const VelSampler& s, float gx, float gy, float hx, float hy, float tdt,
                                            float& ox, float& oy) {
-  const float hd = 0.5f * tdt;
-  float wx, wy; s.vel(s.moved(gx, hd * vx), s.moved(gy, hd * vy), wx, wy);
+  float wx, wy; s.vel(gx - hx, gy - hy, wx, wy);
   ox = s.moved(gx, tdt * wx); oy = s.moved(gy, tdt * wy);
 }
 // sample and the corners' range at one point
@@ -183,8 +183,9 @@ __device__ __forceinline__ int beyond(float gx, float gy, float ox, float oy, in
 // app's plumes at its fixed 2-4 ms steps. Bound by instruction issue and fetch: 12.4 M warp
 // instructions at 256x384 before (every trace from the general sampler, twice; the limits gathered
 // again; two halo cells everywhere, and beyond them four recomputed traces per sample).
-// Now (back to back): 20.1 -> 14.4 us at 256x384, 50 -> 37 at 512x768 (CFL 0.5); 26.7 -> 14.2 at 224x320
-// and 47 -> 29 at 352x512 (3 and 2 ms steps).
+// Now (back to back): 20.1 -> 14.9 us at 256x384, 50 -> 37.7 at 512x768 (CFL 0.5; 0.4 us of each for the bound on
+// displacements, with the half step's shared by both directions); 26.7 -> 14.2 at 224x320 and 47 -> 29 at 352x512
+// (3 and 2 ms steps).
 // Registers for three CTAs of 256 threads per SM (80, no spill in the tile's own path): with 64 and
 // four CTAs 256x384 took 16.1 instead of 14.6 us, 512x768 36.8 instead of 37.1.
 template <int TX, int TY, int H>
@@ -203,7 +204,7 @@ __global__ void __launch_bounds__(TX * TY, TX * TY == 256 ? 3 : 2) k_advect(cons
   const SceneDesc& S = scenes[w.scene];
   if (!S.enabled) return;
   const int nx = S.nx, ny = S.ny, pc = S.pc, pu = S.pu;
-  const float dt = S.P.dt;
+  const float dt = S.P.dt, hd = 0.5f * dt;
   const int x0 = w.tx * TX, y0 = w.ty * TY;
   const int rx0 = x0 - H, ry0 = y0 - H;
 
@@ -224,9 +225,11 @@ __global__ void __launch_bounds__(TX * TY, TX * TY == 256 ? 3 : 2) k_advect(cons
   __syncthreads();
   if (own) {
     const float gx = (float)i + 0.5f, gy = (float)j + 0.5f;
-    float vx, vy, ox, oy;
+    float vx, vy, hx, hy, ox, oy;
+    auto half = [&] { hx = vs.bounded(hd * vx); hy = vs.bounded(hd * vy); };
     vel_cell(vs, i, j, vx, vy);
-    trace_from(vs, gx, gy, vx, vy, dt, ox, oy);
+    half();
+    trace_from(vs, gx, gy, hx, hy, dt, ox, oy);
     {
       float tx, ty;
       const int ci = floor_frac(ox - 0.5f, tx), cj = floor_frac(oy - 0.5f, ty);
@@ -239,22 +242,24 @@ __global__ void __launch_bounds__(TX * TY, TX * TY == 256 ? 3 : 2) k_advect(cons
       ylo = min4(min4(A4, C4), min4(D4, E4)); yhi = max4(max4(A4, C4), max4(D4, E4));
       yh = mix4(mix4(A4, C4, tx), mix4(D4, E4, tx), ty);
     }
-    trace_from(vs, gx, gy, vx, vy, -dt, cbx, cby);
+    trace_from(vs, gx, gy, -hx, -hy, -dt, cbx, cby);
     far = max(far, beyond(cbx, cby, 0.5f, 0.5f, x0, y0, x0 + TX - 1, y0 + TY - 1));
     const int r = (lj + H) * RW + li + H;
     sTh[r] = th; sYh[r] = yh;
     // U face
     vel_uface(vs, i, j, vx, vy);
-    trace_from(vs, (float)i, gy, vx, vy, dt, ox, oy);
+    half();
+    trace_from(vs, (float)i, gy, hx, hy, dt, ox, oy);
     uh = sample_range(vs.u, ox, oy, 0.f, 0.5f, ulo, uhi);
-    trace_from(vs, (float)i, gy, vx, vy, -dt, ubx, uby);
+    trace_from(vs, (float)i, gy, -hx, -hy, -dt, ubx, uby);
     far = max(far, beyond(ubx, uby, 0.f, 0.5f, x0, y0, x0 + TX, y0 + TY - 1));
     sUh[(lj + H) * UW + li + H] = uh;
     // V face
     vel_vface(vs, i, j, vx, vy);
-    trace_from(vs, gx, (float)j, vx, vy, dt, ox, oy);
+    half();
+    trace_from(vs, gx, (float)j, hx, hy, dt, ox, oy);
     vh = sample_range(vs.v, ox, oy, 0.5f, 0.f, vlo, vhi);
-    trace_from(vs, gx, (float)j, vx, vy, -dt, vbx, vby);
+    trace_from(vs, gx, (float)j, -hx, -hy, -dt, vbx, vby);
     far = max(far, beyond(vbx, vby, 0.5f, 0.f, x0, y0, x0 + TX - 1, y0 + TY));
     sVh[(lj + H) * VW + li + H] = vh;
   } else if (i == nx && j < ny) {   // the last faces of a domain that ends inside the tile
@@ -288,7 +293,8 @@ __global__ void __launch_bounds__(TX * TY, TX * TY == 256 ? 3 : 2) k_advect(cons
     if (f == 0) vel_cell(vs, ci, cj, vx, vy);
     else if (f == 1) vel_uface(vs, ci, cj, vx, vy);
     else vel_vface(vs, ci, cj, vx, vy);
-    trace_from(vs, (float)ci + (f == 1 ? 0.f : 0.5f), (float)cj + (f == 2 ? 0.f : 0.5f), vx, vy, dt, ox, oy);
+    const float hx = vs.bounded(hd * vx), hy = vs.bounded(hd * vy);
+    trace_from(vs, (float)ci + (f == 1 ? 0.f : 0.5f), (float)cj + (f == 2 ? 0.f : 0.5f), hx, hy, dt, ox, oy);
     if (f == 0) {
       const int r = (b + H) * RW + a + H;
       sTh[r] = sample(Tf, ox, oy, 0.5f, 0.5f);
